@@ -31,7 +31,8 @@ struct vtlb_ctx {
   // next batch comes in and the last result goes out while the current step computes
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
   cudaEvent_t ev_copy = nullptr;       // ordering between the copy streams and compute
-  uint32_t* d_status = nullptr;        // device status word
+  uint32_t* d_status = nullptr;        // device status word, and (kTicketWord) the block ticket of last_block()
+  static constexpr int kTicketWord = 32;
   void* scratch = nullptr;             // operand-split buffers, partial sums
   size_t scratch_bytes = 0;
   // INT8 pair GEMM, K-split tiles: flags + parked accumulators (kKsplitBytes, allocated with the
@@ -178,6 +179,21 @@ static inline cudaError_t vtlb_launch_early(void (*kern)(KArgs...), dim3 grid, d
   cfg.numAttrs = on ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<Args&&>(args)...);
 }
+
+#ifdef __CUDACC__
+// True in every thread of the CTA that is the last of the grid to get here: it then sees what all the
+// others wrote before.  `ticket` counts the CTAs and wraps to zero by itself, so the next launch on the
+// compute stream finds it reset.  Saves the second launch of a two-stage reduction.
+__device__ __forceinline__ bool vtlb_last_block(uint32_t* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+#endif
 
 static inline bool vtlb_aligned16(const void* p) { return (((uintptr_t)p) & 15u) == 0; }
 static inline size_t vtlb_round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }

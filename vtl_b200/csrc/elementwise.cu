@@ -81,24 +81,59 @@ __device__ __forceinline__ double block_sum(double v, double* smem) {
   return t;  // valid in thread 0
 }
 
+// Second stage of the losses' sums: the CTA that finishes last adds the CTAs' partial sums in a fixed order.
+__device__ __forceinline__ double partials_sum(const double* partial, double* smem) {
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc += __ldcg(partial + i);
+  __syncthreads();  // smem may still be read by the first stage
+  return block_sum(acc, smem);
+}
+
 // dP = p - t (the reference's g*(p-t)/g.size with g = [1]); per-block partial sums
 // of (f32)((f64)d)^2, accumulated in f64.  The reduction is two-stage and has a
-// fixed order, so results are reproducible run to run.
-__global__ void __launch_bounds__(256) mse_partial_kernel(const float* __restrict__ p,
-                                                          const float* __restrict__ t, size_t n,
-                                                          float* __restrict__ dp,
-                                                          double* __restrict__ partial) {
+// fixed order, so results are reproducible run to run.  HBM-bound: 12 bytes per element; with one float
+// per access and a second launch 33.5 M elements took 90 us.
+template <bool VEC>
+__global__ void __launch_bounds__(256) mse_kernel(const float* __restrict__ p, const float* __restrict__ t, size_t n,
+                                                  float* __restrict__ dp, double* __restrict__ partial,
+                                                  uint32_t* ticket, double divisor, float* __restrict__ loss) {
   __shared__ double sm[8];
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   double acc = 0.0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const float d = __fsub_rn(p[i], t[i]);
-    if (dp) dp[i] = d;
+  auto one = [&](float a, float b) {
+    const float d = __fsub_rn(a, b);
     const double dd = (double)d;
     acc += (double)(float)(dd * dd);
+    return d;
+  };
+  const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  if (VEC) {
+    for (size_t i = first; i < n / 4; i += stride) {
+      const float4 a = __ldcs(reinterpret_cast<const float4*>(p) + i), b = __ldcs(reinterpret_cast<const float4*>(t) + i);
+      float4 d;
+      d.x = one(a.x, b.x);
+      d.y = one(a.y, b.y);
+      d.z = one(a.z, b.z);
+      d.w = one(a.w, b.w);
+      if (dp) reinterpret_cast<float4*>(dp)[i] = d;
+    }
+    if (first < n % 4) {
+      const size_t i = n / 4 * 4 + first;
+      const float d = one(p[i], t[i]);
+      if (dp) dp[i] = d;
+    }
+  } else {
+    for (size_t i = first; i < n; i += stride) {
+      const float d = one(p[i], t[i]);
+      if (dp) dp[i] = d;
+    }
   }
   const double s = block_sum(acc, sm);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (!vtlb_last_block(ticket)) return;
+  const double total = partials_sum(partial, sm);
+  if (threadIdx.x == 0) *loss = __fdiv_rn((float)total, (float)divisor);
 }
 // Short inputs: one CTA does both stages in a single launch.
 __global__ void __launch_bounds__(256) mse_short_kernel(const float* __restrict__ p, const float* __restrict__ t,
@@ -118,49 +153,77 @@ __global__ void __launch_bounds__(256) mse_short_kernel(const float* __restrict_
   if (threadIdx.x == 0) *loss = __fdiv_rn((float)s, (float)divisor);
 }
 
-__global__ void __launch_bounds__(256) loss_final_kernel(const double* __restrict__ partial,
-                                                         int nparts, double divisor,
-                                                         int divide_in_f32,
+// Softmax cross-entropy, everything in f64 as in the reference; loss and gradient in one launch.  G lanes
+// share a row (G = 4 to 32 by the class count) and each keeps its NV logits and their exponentials in
+// registers; NV = 0: more than 256 classes, the row is read again (from L1) and exp() taken twice.  A launch
+// is bound by the latency of exp() and the sums: with one thread per row and a second launch for the loss
+// 256 rows took 54 us at 100 classes and 10 us at 10.
+template <int G, int NV>
+__global__ void __launch_bounds__(256) softmax_ce_kernel(const float* __restrict__ x, const float* __restrict__ t, int B,
+                                                         int C, double batch_div, float* __restrict__ dx,
+                                                         double* __restrict__ partial, uint32_t* ticket,
                                                          float* __restrict__ loss) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done from here on
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ double sm[8];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc += partial[i];
-  const double s = block_sum(acc, sm);
-  if (threadIdx.x == 0)
-    *loss = divide_in_f32 ? __fdiv_rn((float)s, (float)divisor) : (float)(s / divisor);
-}
-
-// One thread per row: the class count is small (10 in the configurations this
-// serves) and everything is f64, as in the reference.
-__global__ void __launch_bounds__(128) softmax_ce_kernel(const float* __restrict__ x,
-                                                         const float* __restrict__ t, int B, int C,
-                                                         double batch_div, float* __restrict__ dx,
-                                                         double* __restrict__ partial) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done from here on
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  __shared__ double sm[8];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double li = 0.0;
-  if (i < B) {
-    const float* xi = x + (size_t)i * C;
-    const float* ti = t + (size_t)i * C;
-    double mx = (double)xi[0];
-    for (int c = 1; c < C; ++c) mx = fmax(mx, (double)xi[c]);
-    double se = 0.0;
-    for (int c = 0; c < C; ++c) se += exp((double)xi[c] - mx);
-    double dot = 0.0;
-    for (int c = 0; c < C; ++c) dot += (double)ti[c] * (double)xi[c];
-    li = log(se) + mx - dot;
-    if (dx)
-      for (int c = 0; c < C; ++c) {
-        const double smx = exp((double)xi[c] - mx) / se;
-        dx[(size_t)i * C + c] = (float)((smx - (double)ti[c]) / batch_div);
+  const int row = blockIdx.x * (256 / G) + threadIdx.x / G, gl = threadIdx.x % G;
+  const bool live = row < B;  // the lanes of a row agree; nobody leaves before the shuffles
+  const float* xi = x + (size_t)(live ? row : 0) * C;
+  const float* ti = t + (size_t)(live ? row : 0) * C;
+  auto group_sum = [](double v) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  double mx = -INFINITY, se = 0.0, dot = 0.0, li;
+  if constexpr (NV > 0) {
+    float xv[NV], tv[NV];
+    double e[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int c = gl + j * G;
+      xv[j] = c < C ? xi[c] : -INFINITY;
+      tv[j] = c < C ? ti[c] : 0.0f;
+      mx = fmax(mx, (double)xv[j]);
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const bool in = gl + j * G < C;
+      e[j] = in ? exp((double)xv[j] - mx) : 0.0;
+      se += e[j];
+      if (in) dot += (double)tv[j] * (double)xv[j];
+    }
+    se = group_sum(se);
+    dot = group_sum(dot);
+    if (dx && live) {
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const int c = gl + j * G;
+        if (c < C) dx[(size_t)row * C + c] = (float)((e[j] / se - (double)tv[j]) / batch_div);
       }
+    }
+  } else {
+    for (int c = gl; c < C; c += G) mx = fmax(mx, (double)xi[c]);
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int c = gl; c < C; c += G) {
+      se += exp((double)xi[c] - mx);
+      dot += (double)ti[c] * (double)xi[c];
+    }
+    se = group_sum(se);
+    dot = group_sum(dot);
+    if (dx && live)
+      for (int c = gl; c < C; c += G)
+        dx[(size_t)row * C + c] = (float)((exp((double)xi[c] - mx) / se - (double)ti[c]) / batch_div);
   }
+  li = live && gl == 0 ? log(se) + mx - dot : 0.0;
   const double s = block_sum(li, sm);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (!vtlb_last_block(ticket)) return;
+  const double total = partials_sum(partial, sm);
+  if (threadIdx.x == 0) *loss = (float)(total / batch_div);
 }
 
 }  // namespace
@@ -222,11 +285,10 @@ VTLB_API int vtlb_mse_fwd_bwd_f32(vtlb_ctx* ctx, const void* d_P, const void* d_
   void* scr = nullptr;
   int rc = vtlb_scratch(ctx, (size_t)blocks * sizeof(double), &scr);
   if (rc) return rc;
-  mse_partial_kernel<<<blocks, 256, 0, ctx->stream>>>((const float*)d_P, (const float*)d_T, n,
-                                                      (float*)d_dP_or_null, (double*)scr);
-  VTLB_LAUNCHED(ctx);
-  VTLB_CUDA(ctx, vtlb_launch_early(loss_final_kernel, dim3(1), dim3(256), 0, ctx->stream, (const double*)scr, blocks,
-                                   (double)n_div, 1, (float*)d_loss));
+  const bool vec = vtlb_aligned16(d_P) && vtlb_aligned16(d_T) && (!d_dP_or_null || vtlb_aligned16(d_dP_or_null));
+  VTLB_CUDA(ctx, vtlb_launch_early(vec ? mse_kernel<true> : mse_kernel<false>, dim3(blocks), dim3(256), 0, ctx->stream,
+                                   (const float*)d_P, (const float*)d_T, n, (float*)d_dP_or_null, (double*)scr,
+                                   ctx->d_status + vtlb_ctx::kTicketWord, (double)n_div, (float*)d_loss));
   VTLB_LAUNCHED(ctx);
   return VTLB_OK;
 }
@@ -237,15 +299,17 @@ VTLB_API int vtlb_softmax_ce_fwd_bwd_f32(vtlb_ctx* ctx, const void* d_X, const v
   if (B <= 0 || C <= 0 || batch_div <= 0)
     return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_softmax_ce_fwd_bwd_f32: bad shape B=%d C=%d div=%d", B, C, batch_div);
   if (!d_X || !d_T || !d_loss) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_softmax_ce_fwd_bwd_f32: null pointer");
-  const int blocks = (B + 127) / 128;
+  const int lanes = C <= 4 ? 4 : C <= 8 ? 8 : C <= 16 ? 16 : 32, rows_per_block = 256 / lanes;
+  const int blocks = (B + rows_per_block - 1) / rows_per_block;
   void* scr = nullptr;
   int rc = vtlb_scratch(ctx, (size_t)blocks * sizeof(double), &scr);
   if (rc) return rc;
-  VTLB_CUDA(ctx, vtlb_launch_early(softmax_ce_kernel, dim3(blocks), dim3(128), 0, ctx->stream, (const float*)d_X,
-                                   (const float*)d_T, B, C, (double)batch_div, (float*)d_dX_or_null, (double*)scr));
-  VTLB_LAUNCHED(ctx);
-  VTLB_CUDA(ctx, vtlb_launch_early(loss_final_kernel, dim3(1), dim3(256), 0, ctx->stream, (const double*)scr, blocks,
-                                   (double)batch_div, 0, (float*)d_loss));
+  auto kern = C <= 4 ? softmax_ce_kernel<4, 1> : C <= 8 ? softmax_ce_kernel<8, 1> : C <= 16 ? softmax_ce_kernel<16, 1>
+              : C <= 32 ? softmax_ce_kernel<32, 1> : C <= 64 ? softmax_ce_kernel<32, 2>
+              : C <= 128 ? softmax_ce_kernel<32, 4> : C <= 256 ? softmax_ce_kernel<32, 8> : softmax_ce_kernel<32, 0>;
+  VTLB_CUDA(ctx, vtlb_launch_early(kern, dim3(blocks), dim3(256), 0, ctx->stream, (const float*)d_X, (const float*)d_T,
+                                   B, C, (double)batch_div, (float*)d_dX_or_null, (double*)scr,
+                                   ctx->d_status + vtlb_ctx::kTicketWord, (float*)d_loss));
   VTLB_LAUNCHED(ctx);
   return VTLB_OK;
 }

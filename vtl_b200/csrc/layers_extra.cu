@@ -134,25 +134,38 @@ __global__ void __launch_bounds__(256) bn_colsum_kernel(const float* __restrict_
   const int r0 = s * per, r1 = min(B, r0 + per);
   const double mu = MODE == BN_SUM ? 0.0 : mean[c];
   double acc = 0.0;
-  for (int r = r0; r < r1; ++r) {
-    const double v = (double)a[(size_t)r * F + c];
-    if (MODE == BN_SUM) acc = __dadd_rn(acc, v);
-    if (MODE == BN_SQDIFF) {
-      const double dlt = __dsub_rn(v, mu);
-      acc = __dadd_rn(acc, __dmul_rn(dlt, dlt));
+  constexpr int U = 8;  // rows whose loads are in flight together: the sum itself is a serial chain
+  for (int r = r0; r < r1; r += U) {
+    float va[U], vb[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int rr = min(r + u, r1 - 1);
+      va[u] = a[(size_t)rr * F + c];
+      vb[u] = MODE == BN_PROD_CENTERED ? b[(size_t)rr * F + c] : 0.0f;
     }
-    if (MODE == BN_PROD_CENTERED) acc = __dadd_rn(acc, __dmul_rn(v, __dsub_rn((double)b[(size_t)r * F + c], mu)));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (r + u >= r1) break;
+      const double v = (double)va[u];
+      if (MODE == BN_SUM) acc = __dadd_rn(acc, v);
+      if (MODE == BN_SQDIFF) {
+        const double dlt = __dsub_rn(v, mu);
+        acc = __dadd_rn(acc, __dmul_rn(dlt, dlt));
+      }
+      if (MODE == BN_PROD_CENTERED) acc = __dadd_rn(acc, __dmul_rn(v, __dsub_rn((double)vb[u], mu)));
+    }
   }
   partial[(size_t)s * F + c] = acc;
 }
-// out[c] = (sum over slices) / divisor
+// out[c] = (sum over slices) / divisor; sum_out[c] (may be null) = the sum itself
 __global__ void bn_colsum_final_kernel(const double* __restrict__ partial, int S, int F, double divisor,
-                                       double* __restrict__ out) {
+                                       double* __restrict__ out, double* __restrict__ sum_out) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= F) return;
   double t = 0.0;
   for (int s = 0; s < S; ++s) t = __dadd_rn(t, partial[(size_t)s * F + c]);
   out[c] = __ddiv_rn(t, divisor);
+  if (sum_out) sum_out[c] = t;
 }
 
 // y = gamma * (x - mean) / sqrt(var + eps) + beta in f64; also the f32 batch statistics and the
@@ -225,6 +238,124 @@ __global__ void widen_kernel(const float* __restrict__ a, int n, double* __restr
   if (i < n) out[i] = (double)a[i];
 }
 
+// ---- batches of at most kBnFusedRows rows: one launch
+// Bound by launches and latency, not bytes (256 x 512: 0.5 MB).  The sliced path above needs six launches
+// in training and five backward and puts 256 rows on eight CTAs, each a serial chain of loads and f64 adds
+// (89 us forward, 72 us backward, measured one by one); here a CTA owns 8 features (whole 32-byte sectors),
+// keeps every row of them in registers and takes the sums in two shuffle steps and one pass over eight
+// partial sums.  Longer batches stay on the sliced path: their rows do not fit the registers of a CTA.
+constexpr int kBnFusedRows = 1024;
+
+// Sum over the 32 row lanes of each of the CTA's 8 columns, in a fixed order; every thread gets its column's.
+__device__ __forceinline__ double bn_column_sum(double v, double (*sm)[8]) {
+  v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
+  v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 16));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __syncthreads();  // the previous use of sm is over
+  if (lane < 8) sm[warp][lane] = v;
+  __syncthreads();
+  double t = sm[0][lane & 7];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) t = __dadd_rn(t, sm[w][lane & 7]);
+  return t;
+}
+
+template <int VPT>
+__global__ void __launch_bounds__(256) bn_train_fused_kernel(const float* __restrict__ x, int B, int F,
+                                                             const float* __restrict__ gamma,
+                                                             const float* __restrict__ beta, double eps,
+                                                             float* __restrict__ y, float* __restrict__ mean_out,
+                                                             float* __restrict__ var_out, float* running_mean,
+                                                             float* running_var, double momentum) {
+  __shared__ double sm[8][8];
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early: the kernel in front is done from here on
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int c = blockIdx.x * 8 + (threadIdx.x & 7), rl = threadIdx.x >> 3;
+  const bool col = c < F;
+  float v[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int r = rl + 32 * i;
+    v[i] = col && r < B ? x[(size_t)r * F + c] : 0.0f;
+  }
+  double acc = 0.0;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (rl + 32 * i < B) acc = __dadd_rn(acc, (double)v[i]);
+  const double mean = __ddiv_rn(bn_column_sum(acc, sm), (double)B);
+  acc = 0.0;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (rl + 32 * i < B) {
+      const double d = __dsub_rn((double)v[i], mean);
+      acc = __dadd_rn(acc, __dmul_rn(d, d));
+    }
+  const double var = __ddiv_rn(bn_column_sum(acc, sm), (double)B);
+  if (!col) return;
+  const double std = __dsqrt_rn(__dadd_rn(var, eps)), gam = (double)gamma[c], bet = (double)beta[c];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int r = rl + 32 * i;
+    if (r < B) y[(size_t)r * F + c] = (float)__dadd_rn(__dmul_rn(gam, __ddiv_rn(__dsub_rn((double)v[i], mean), std)), bet);
+  }
+  if (rl == 0) {
+    const float m = (float)mean, w = (float)var;
+    mean_out[c] = m;
+    var_out[c] = w;
+    if (running_mean) {
+      const double om = __dsub_rn(1.0, momentum);
+      running_mean[c] = (float)__dadd_rn(__dmul_rn(momentum, (double)m), __dmul_rn(om, (double)running_mean[c]));
+      running_var[c] = (float)__dadd_rn(__dmul_rn(momentum, (double)w), __dmul_rn(om, (double)running_var[c]));
+    }
+  }
+}
+
+template <int VPT>
+__global__ void __launch_bounds__(256) bn_bwd_fused_kernel(const float* __restrict__ g, const float* __restrict__ x,
+                                                           int B, int F, const float* __restrict__ gamma,
+                                                           const float* __restrict__ mean,
+                                                           const float* __restrict__ var, double eps,
+                                                           float* __restrict__ dx, float* __restrict__ dgamma,
+                                                           float* __restrict__ dbeta) {
+  __shared__ double sm[8][8];
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early: the kernel in front is done from here on
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int c = blockIdx.x * 8 + (threadIdx.x & 7), rl = threadIdx.x >> 3;
+  const bool col = c < F;
+  float v[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int r = rl + 32 * i;
+    v[i] = col && r < B ? g[(size_t)r * F + c] : 0.0f;
+  }
+  double acc = 0.0;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (rl + 32 * i < B) acc = __dadd_rn(acc, (double)v[i]);
+  const double gsum = bn_column_sum(acc, sm);
+  const double std = __dsqrt_rn(__dadd_rn(col ? (double)var[c] : 1.0, eps));
+  if (dx && col) {
+    const double gmean = __ddiv_rn(gsum, (double)B), gam = (double)gamma[c];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int r = rl + 32 * i;
+      if (r < B) dx[(size_t)r * F + c] = (float)__ddiv_rn(__dmul_rn(gam, __dsub_rn((double)v[i], gmean)), std);
+    }
+  }
+  if (dgamma) {
+    const double mu = col ? (double)mean[c] : 0.0;
+    acc = 0.0;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int r = rl + 32 * i;
+      if (col && r < B) acc = __dadd_rn(acc, __dmul_rn((double)v[i], __dsub_rn((double)x[(size_t)r * F + c], mu)));
+    }
+    const double gprod = bn_column_sum(acc, sm);
+    if (col && rl == 0) dgamma[c] = (float)__ddiv_rn(gprod, std);
+  }
+  if (dbeta && col && rl == 0) dbeta[c] = (float)gsum;
+}
+
 int bn_slices(vtlb_ctx* ctx, int B, int F) {
   const int col_blocks = (F + 255) / 256;
   int S = (4 * ctx->sm_count + col_blocks - 1) / col_blocks;
@@ -234,10 +365,10 @@ int bn_slices(vtlb_ctx* ctx, int B, int F) {
 
 template <int MODE>
 int bn_colsum(vtlb_ctx* ctx, const float* a, const float* b, const double* mean, int B, int F, double divisor,
-              double* partial, int S, double* out) {
+              double* partial, int S, double* out, double* sum_out = nullptr) {
   bn_colsum_kernel<MODE><<<dim3((F + 255) / 256, S), 256, 0, ctx->stream>>>(a, b, mean, B, F, partial);
   VTLB_LAUNCHED(ctx);
-  bn_colsum_final_kernel<<<(F + 255) / 256, 256, 0, ctx->stream>>>(partial, S, F, divisor, out);
+  bn_colsum_final_kernel<<<(F + 255) / 256, 256, 0, ctx->stream>>>(partial, S, F, divisor, out, sum_out);
   VTLB_LAUNCHED(ctx);
   return VTLB_OK;
 }
@@ -333,6 +464,20 @@ VTLB_API int vtlb_batchnorm1d_train_f32(vtlb_ctx* ctx, const void* d_x, int B, i
   if (!d_x || !d_gamma || !d_beta || !d_y || !d_batch_mean || !d_batch_var ||
       (!d_running_mean_or_null) != (!d_running_var_or_null))
     return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_batchnorm1d_train_f32: null pointer");
+  if (B <= kBnFusedRows) {
+#define VTLB_BN_TRAIN(VPT)                                                                                       \
+  VTLB_CUDA(ctx, vtlb_launch_early(bn_train_fused_kernel<VPT>, dim3((F + 7) / 8), dim3(256), 0, ctx->stream,       \
+                                   (const float*)d_x, B, F, (const float*)d_gamma, (const float*)d_beta, eps,      \
+                                   (float*)d_y, (float*)d_batch_mean, (float*)d_batch_var,                         \
+                                   (float*)d_running_mean_or_null, (float*)d_running_var_or_null, momentum))
+    if (B <= 128) VTLB_BN_TRAIN(4);
+    else if (B <= 256) VTLB_BN_TRAIN(8);
+    else if (B <= 512) VTLB_BN_TRAIN(16);
+    else VTLB_BN_TRAIN(32);
+#undef VTLB_BN_TRAIN
+    VTLB_LAUNCHED(ctx);
+    return VTLB_OK;
+  }
   const int S = bn_slices(ctx, B, F);
   void* scr = nullptr;
   int rc = vtlb_scratch(ctx, ((size_t)S * F + 2 * (size_t)F) * sizeof(double), &scr);
@@ -375,6 +520,20 @@ VTLB_API int vtlb_batchnorm1d_bwd_f32(vtlb_ctx* ctx, const void* d_g, const void
   if (B <= 0 || F <= 0) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_batchnorm1d_bwd_f32: bad shape B=%d F=%d", B, F);
   if (!d_g || !d_x || !d_gamma || !d_batch_mean || !d_batch_var)
     return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_batchnorm1d_bwd_f32: null pointer");
+  if (B <= kBnFusedRows) {
+#define VTLB_BN_BWD(VPT)                                                                                         \
+  VTLB_CUDA(ctx, vtlb_launch_early(bn_bwd_fused_kernel<VPT>, dim3((F + 7) / 8), dim3(256), 0, ctx->stream,         \
+                                   (const float*)d_g, (const float*)d_x, B, F, (const float*)d_gamma,              \
+                                   (const float*)d_batch_mean, (const float*)d_batch_var, eps,                     \
+                                   (float*)d_dx_or_null, (float*)d_dgamma_or_null, (float*)d_dbeta_or_null))
+    if (B <= 128) VTLB_BN_BWD(4);
+    else if (B <= 256) VTLB_BN_BWD(8);
+    else if (B <= 512) VTLB_BN_BWD(16);
+    else VTLB_BN_BWD(32);
+#undef VTLB_BN_BWD
+    VTLB_LAUNCHED(ctx);
+    return VTLB_OK;
+  }
   const int S = bn_slices(ctx, B, F);
   void* scr = nullptr;
   int rc = vtlb_scratch(ctx, ((size_t)S * F + 4 * (size_t)F) * sizeof(double), &scr);
@@ -385,8 +544,7 @@ VTLB_API int vtlb_batchnorm1d_bwd_f32(vtlb_ctx* ctx, const void* d_g, const void
   double* gprod = gmean + F;
   double* mean64 = gprod + F;
   const float* g = (const float*)d_g;
-  if ((rc = bn_colsum<BN_SUM>(ctx, g, nullptr, nullptr, B, F, 1.0, partial, S, gsum))) return rc;
-  if ((rc = bn_colsum<BN_SUM>(ctx, g, nullptr, nullptr, B, F, (double)B, partial, S, gmean))) return rc;
+  if ((rc = bn_colsum<BN_SUM>(ctx, g, nullptr, nullptr, B, F, (double)B, partial, S, gmean, gsum))) return rc;
   if (d_dx_or_null) {
     bn_bwd_apply_kernel<<<ex_grid(ctx, (size_t)B * F, 1024), 256, 0, ctx->stream>>>(
         g, B, F, (const float*)d_gamma, (const float*)d_batch_var, eps, gmean, (float*)d_dx_or_null);
