@@ -100,6 +100,28 @@ __device__ __forceinline__ void stage_and_store(uint32_t stg, const CUtensorMap*
   }
 }
 
+// The same chunk where the output's row pitch is no multiple of 16 bytes, which TMA cannot describe: the warp
+// turns it round through its staging tile and writes one row per instruction, 32 consecutive words.  Each lane
+// storing its own row instead touches 32 sectors per 4-byte store: that bounded the 999 x 3001 x 2047 INT8 GEMM
+// (with its quantisation 49.9 us a pass; 24.6 us this way).
+__device__ __forceinline__ void stage_and_store_rows(uint32_t stg, uint32_t* __restrict__ out, int ldo, int lane,
+                                                     int row0, int col0, const uint32_t (&v)[32], int M, int N) {
+  const uint32_t rowaddr = stg + lane * 128;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    ptx::st_shared_v4(rowaddr + (((uint32_t)j ^ ((uint32_t)lane & 7u)) << 4), v[4 * j], v[4 * j + 1],
+                      v[4 * j + 2], v[4 * j + 3]);
+  __syncwarp();
+  const int rows = M - row0 < 32 ? M - row0 : 32;
+  if (col0 + lane < N) {
+    uint32_t* o = out + (size_t)row0 * ldo + col0 + lane;
+    const uint32_t src = stg + ((uint32_t)lane & 3u) * 4u, quad = (uint32_t)lane >> 2;
+#pragma unroll 8
+    for (int r = 0; r < rows; ++r)
+      o[(size_t)r * ldo] = ptx::ld_shared_u32(src + (uint32_t)r * 128u + ((quad ^ ((uint32_t)r & 7u)) << 4));
+  }
+}
+
 // x = hi + lo + O(2^-22 |x|), both representable in TF32 (the operand split of the 3xTF32 products).
 __device__ __forceinline__ uint32_t tf32_hi_bits(uint32_t x) {
   uint32_t r;
@@ -398,18 +420,26 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, const Epi epi, int M, int N, 
       const int kb_end = kb_begin + kb_per_split < total_kb ? kb_begin + kb_per_split : total_kb;
       const int row0 = m0 + q * 32;
       if constexpr (KIND == KIND_I8) {
+        // scales and bias are fetched before the wait, one column per lane, and handed round by shuffles
+        const typename Epi::Pre pre = epi.prefetch(row0 + lane, n0 + half * 32 + lane, M, N);
         ok = ptx::mbar_wait_bounded(tfull_bar(acc), acc_phase, abort_flag, WAIT_LIMIT_NS);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         ptx::tc_fence_after();
-#pragma unroll 1
-        for (int c = half; c < BN / 32; c += 2) {
+        float row_amax = 0.0f;
+#pragma unroll
+        for (int cc = 0; cc < BN / 64; ++cc) {
+          const int col0 = n0 + (2 * cc + half) * 32;
           uint32_t v[32];
-          ptx::tmem_ld_32x32(lane_base + acc * BN + c * 32, v);
+          ptx::tmem_ld_32x32(lane_base + acc * BN + (2 * cc + half) * 32, v);
           ptx::tmem_wait_ld();
-          epilogue_chunk(epi, tm, stg, lane, row0, n0 + c * 32, v, M, N, split);
+          epi.transform_pre(pre, cc, v);
+          row_amax = fmaxf(row_amax, epi.chunk_amax(col0, v, N));
+          if (epi.tma) stage_and_store(stg, &tm.out[0], lane, row0, col0, v, M, N);
+          else stage_and_store_rows(stg, epi.out_words(), epi.out_pitch(), lane, row0, col0, v, M, N);
           __syncwarp();
         }
+        epi.commit_amax(row0 + lane, M, row_amax);
         ptx::tc_fence_before();
         ptx::mbar_arrive(tempty_bar(acc));
         acc ^= 1u;

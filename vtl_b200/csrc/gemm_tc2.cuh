@@ -378,9 +378,7 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
         // Per-row and per-column operands of the epilogue (scales, bias) are fetched before the
         // wait for the accumulator, one column per lane, and handed round by shuffles later:
         // their latency would otherwise sit in front of every 32-column chunk.
-        const bool fast = epi.tma != 0;
-        typename Epi::Pre pre;
-        if (fast) pre = epi.prefetch(row0 + lane, n0 + half * 32 + lane, M, N);
+        const typename Epi::Pre pre = epi.prefetch(row0 + lane, n0 + half * 32 + lane, M, N);
         ok = ptx::mbar_wait_bounded(tfull_bar(acc), acc_phase, abort_flag, WAIT_LIMIT_NS);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -395,7 +393,7 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
           if (!ok) break;
         }
         float row_amax = 0.0f;
-        auto do_chunk = [&](int cc, bool use_pre) {
+        auto do_chunk = [&](int cc, bool tma) {
           const int c = 2 * cc + half;
           uint32_t v[32];
           ptx::tmem_ld_32x32(lane_base + acc * BN2 + c * 32, v);
@@ -409,24 +407,21 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
 #pragma unroll
               for (int j = 0; j < 32; ++j) v[j] += __ldcg(pc + j * 32);
             }
-            if (use_pre) {
-              epi.transform_pre(pre, cc, v);
-              row_amax = fmaxf(row_amax, epi.chunk_amax(n0 + c * 32, v, N));  // one atomic per warp and tile
-              gemm::stage_and_store(stg, &tm.out[0], lane, row0, n0 + c * 32, v, M, N);
-            } else {
-              gemm::epilogue_chunk(epi, tm, stg, lane, row0, n0 + c * 32, v, M, N, 0);
-            }
+            epi.transform_pre(pre, cc, v);
+            row_amax = fmaxf(row_amax, epi.chunk_amax(n0 + c * 32, v, N));  // one atomic per warp and tile
+            if (tma) gemm::stage_and_store(stg, &tm.out[0], lane, row0, n0 + c * 32, v, M, N);
+            else gemm::stage_and_store_rows(stg, epi.out_words(), epi.out_pitch(), lane, row0, n0 + c * 32, v, M, N);
           }
           __syncwarp();
         };
-        if (fast) {
+        if (epi.tma != 0) {
 #pragma unroll
           for (int cc = 0; cc < BN2 / 64; ++cc) do_chunk(cc, true);
         } else {
-#pragma unroll 1
+#pragma unroll
           for (int cc = 0; cc < BN2 / 64; ++cc) do_chunk(cc, false);
         }
-        if (fast && kh != 0) epi.commit_amax(row0 + lane, M, row_amax);
+        if (kh != 0) epi.commit_amax(row0 + lane, M, row_amax);
         ptx::tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa(tempty_bar(acc), 0));

@@ -165,32 +165,20 @@ __global__ void __launch_bounds__(256) row_absmax_kernel(const float* __restrict
 }
 
 // ---------------------------------------------------------------- epilogues
+// What the INT8 kernels' epilogue warps ask of a functor: prefetch() before the wait for the accumulator,
+// transform_pre() per 32-column chunk in registers, the row maxima, and where the words go when TMA cannot
+// store them (`tma` = 0: N % 4 != 0).
 struct EpiStoreI32 {
-  static constexpr bool kTmaCapable = true;
   int32_t* C;
   int ldc;
-  int tma;  // store through the output tensor map (tm.out[0]) instead of per-thread stores
-  __device__ __forceinline__ bool transform(int, int, uint32_t (&)[32], int, int) const { return false; }
-  __device__ __forceinline__ void activate(uint32_t (&)[32]) const {}
+  int tma;  // store through the output tensor map (tm.out[0])
   struct Pre {};  // nothing to fetch ahead of the accumulator
   __device__ __forceinline__ Pre prefetch(int, int, int, int) const { return Pre{}; }
   __device__ __forceinline__ void transform_pre(const Pre&, int, uint32_t (&)[32]) const {}
   __device__ __forceinline__ float chunk_amax(int, const uint32_t (&)[32], int) const { return 0.0f; }
   __device__ __forceinline__ void commit_amax(int, int, float) const {}
-  __device__ __forceinline__ void operator()(int row, int col0, const uint32_t (&v)[32], int M,
-                                             int N, int /*split*/) const {
-    if (row >= M) return;
-    int32_t* c = C + (size_t)row * ldc + col0;
-    if (col0 + 32 <= N && (ldc & 3) == 0) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<int4*>(c + j) = make_int4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (col0 + j < N) c[j] = (int32_t)v[j];
-    }
-  }
+  __device__ __forceinline__ uint32_t* out_words() const { return reinterpret_cast<uint32_t*>(C); }
+  __device__ __forceinline__ int out_pitch() const { return ldc; }
 };
 
 __device__ __forceinline__ float dequant1(uint32_t acc, float sa, float sw, float bias,
@@ -203,7 +191,6 @@ __device__ __forceinline__ float dequant1(uint32_t acc, float sa, float sw, floa
 }
 
 struct EpiDequant {
-  static constexpr bool kTmaCapable = true;
   float* Y;
   const float* sa;
   const float* sw;
@@ -227,33 +214,11 @@ struct EpiDequant {
   __device__ __forceinline__ void commit_amax(int row, int M, float m) const {
     if (amax != nullptr && row < M) atomicMax(reinterpret_cast<int*>(amax + row), __float_as_int(m));
   }
-  __device__ __forceinline__ void note_amax(int row, int col0, const uint32_t (&v)[32], int M, int N) const {
-    commit_amax(row, M, chunk_amax(col0, v, N));
-  }
-  // dequantises the chunk in registers; rows and columns past the edge yield values the
-  // clipped TMA store never writes
-  __device__ __forceinline__ bool transform(int row, int col0, uint32_t (&v)[32], int M, int N) const {
-    const float s = row < M ? sa[row] : 0.0f;
-    const bool hb = bias != nullptr;
-#pragma unroll
-    for (int j = 0; j < 32; j += 4) {
-      float4 w4 = make_float4(0.f, 0.f, 0.f, 0.f), b4 = w4;
-      if (col0 + j < N) {
-        w4 = __ldg(reinterpret_cast<const float4*>(sw + col0 + j));
-        if (hb) b4 = __ldg(reinterpret_cast<const float4*>(bias + col0 + j));
-      }
-      v[j] = __float_as_uint(dequant1(v[j], s, w4.x, b4.x, hb, relu));
-      v[j + 1] = __float_as_uint(dequant1(v[j + 1], s, w4.y, b4.y, hb, relu));
-      v[j + 2] = __float_as_uint(dequant1(v[j + 2], s, w4.z, b4.z, hb, relu));
-      v[j + 3] = __float_as_uint(dequant1(v[j + 3], s, w4.w, b4.w, hb, relu));
-    }
-    note_amax(row, col0, v, M, N);
-    return false;
-  }
-  __device__ __forceinline__ void activate(uint32_t (&)[32]) const {}
-  // The same dequantisation with its operands fetched ahead (CTA-pair kernel): this lane's row
-  // scale, and for each of the warp's four 32-column chunks (64 columns apart) the weight scale
-  // and bias of ONE column, `col` being this lane's column in the first chunk.
+  __device__ __forceinline__ uint32_t* out_words() const { return reinterpret_cast<uint32_t*>(Y); }
+  __device__ __forceinline__ int out_pitch() const { return ldy; }
+  // The operands of the dequantisation, fetched ahead: this lane's row scale, and for each of the
+  // warp's 32-column chunks (64 columns apart) the weight scale and bias of ONE column, `col` being
+  // this lane's column in the first chunk.
   struct Pre {
     float s;
     float w[4], b[4];
@@ -276,30 +241,6 @@ struct EpiDequant {
       const float w = __shfl_sync(0xffffffffu, p.w[cc], j);
       const float b = __shfl_sync(0xffffffffu, p.b[cc], j);
       v[j] = __float_as_uint(dequant1(v[j], p.s, w, b, hb, relu));
-    }
-  }
-  __device__ __forceinline__ void operator()(int row, int col0, const uint32_t (&v)[32], int M,
-                                             int N, int /*split*/) const {
-    if (row >= M) return;
-    const float s = sa[row];
-    float* y = Y + (size_t)row * ldy + col0;
-    const bool hb = bias != nullptr;
-    uint32_t o[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      o[j] = col0 + j < N ? __float_as_uint(dequant1(v[j], s, __ldg(sw + col0 + j), hb ? __ldg(bias + col0 + j) : 0.0f,
-                                                      hb, relu))
-                          : 0u;
-    note_amax(row, col0, o, M, N);
-    if (col0 + 32 <= N && (ldy & 3) == 0) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<float4*>(y + j) = make_float4(__uint_as_float(o[j]), __uint_as_float(o[j + 1]),
-                                                        __uint_as_float(o[j + 2]), __uint_as_float(o[j + 3]));
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (col0 + j < N) y[j] = __uint_as_float(o[j]);
     }
   }
 };
