@@ -28,6 +28,32 @@ def test_rows_that_tma_cannot_store(dev, M, N, K, relu):
     _check(dev, M, N, K, relu)
 
 
+@pytest.mark.parametrize("M,N,K,relu", [
+    (1, 4097, 272, False), (1, 28672, 128, True),          # dp4a kernel: row maxima over one and several channels a warp
+    (2, 130, 2048, False), (16, 128, 4096, True),          # K over four CTAs, one tile
+    (8, 19073, 256, True), (17, 18945, 144, False), (33, 28672, 256, True),  # more tiles than SMs
+    (64, 38017, 128, False),                               # more tiles than two to an SM
+    (65, 18945, 144, True), (128, 18944, 128, False),      # above 64 rows: the general kernel, and one wave
+])
+def test_few_rows_and_their_maxima(dev, M, N, K, relu):
+    _check(dev, M, N, K, relu)
+
+
+@pytest.mark.parametrize("M,K", [(1, 8208), (3, 28672), (2, 12293), (513, 8196)])
+def test_long_rows_quantised_in_pieces(dev, orc, M, K):
+    A = np.random.default_rng(K).standard_normal((M, K)).astype(np.float32)
+    amax = np.abs(A).max(axis=1)
+    amax[0] = 0.0  # a maximum of zero: scale 0, codes 0
+    dA, dM = dev.to_device(A), dev.to_device(amax)
+    dQ, dS = dev.zeros((M, dev.i8_ld(K)), np.int8), dev.empty((M,), np.float32)
+    dev.quant_rows_i8(dA, M, K, dQ, dS, dM)
+    q_ref, s_ref = orc.quant_rows_i8_with_amax(A, amax)
+    assert np.array_equal(dQ.numpy()[:, :K], q_ref)
+    assert np.array_equal(dS.numpy().view(np.uint32), s_ref.view(np.uint32))
+    for b in (dA, dM, dQ, dS):
+        b.free()
+
+
 def _check(dev, M, N, K, relu):
     rng = np.random.default_rng(M + 3 * N + 7 * K)
     ld = dev.i8_ld(K)

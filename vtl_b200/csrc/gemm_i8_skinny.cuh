@@ -16,7 +16,14 @@
 //     peer's memory after the barrier, so a CTA may leave as soon as it is done; the barrier
 //     that guarantees every peer has started before it is written to is entered at the top
 //     and only waited for after the K loop.
-// One tile per CTA (grid = tiles * S); warp 0 = TMA producer, warp 1 = MMA issuer and owner
+// One tile per CTA (grid = tiles * S).  Up to 64 rows a CTA keeps to half of an SM's shared memory, so that two
+// are resident and any number of tiles streams the weights: 28672 channels are 224 tiles on 148 SMs, and one CTA
+// per SM would leave half of the SMs idle in the second wave, while an SM with two tiles simply draws twice the
+// bandwidth (8 rows, 28672 x 8192: 67.2 us in the general kernel, 42 us here; the weights alone take 36 us).
+// Row maxima for the next layer's quantisation come out of part 2, folded by the CTA that finishes last: eight
+// rows through four layers 8192 - 28672 took 260.8 us, now 180 us (of them 144 us for 0.94 GB of weights).
+// With 65 to 128 rows the landing zone and the operand tiles need a whole SM: one wave of tiles only.
+// warp 0 = TMA producer, warp 1 = MMA issuer and owner
 // of the tensor memory, warps 2..5 = epilogue.  Waits are bounded as in gemm_tc.cuh and both
 // cluster barriers are reached on every path.
 #pragma once
@@ -31,12 +38,27 @@ namespace skinny {
 
 constexpr int BNCH = 128;                      // output channels per tile = TMEM lanes
 constexpr uint32_t W_TILE = BNCH * 128;        // 16 KB of weights per stage
-constexpr uint32_t RING_BYTES = 128 * 1024;    // operand ring
-constexpr uint32_t LZ_BYTES = 64 * 1024;       // landing zone: [source CTA][owned row][128 channels] int32
-constexpr int MAX_STAGES = 8;
+constexpr int MAX_STAGES = 6;
 constexpr int NUM_THREADS = 192;
-constexpr uint32_t BARS_OFF = RING_BYTES + LZ_BYTES;
-constexpr uint32_t SMEM_TOTAL = BARS_OFF + 8 * (2 * MAX_STAGES + 1) + 16 + 1024;
+constexpr uint32_t BARS_BYTES = 8 * (2 * MAX_STAGES + 1) + 16;
+// Shared memory: the operand ring, the landing zone ([source CTA][owned row][128 channels] int32, MN rows in
+// all), the barriers, and 1 KB to align the ring.
+constexpr uint32_t HALF_SM = 112 * 1024;       // two of these (and 1 KB each for the system) fit an SM's 228 KB
+constexpr uint32_t WHOLE_SM = 224 * 1024;
+constexpr int kHalfMaxMN = 64;                 // rows up to which a CTA keeps to half of an SM
+__host__ __device__ constexpr uint32_t stage_bytes(int MN) { return W_TILE + (uint32_t)MN * 128u; }
+__host__ __device__ constexpr uint32_t lz_bytes(int MN) { return (uint32_t)MN * 512u; }
+__host__ __device__ constexpr int num_stages(int MN) {
+  const uint32_t room = (MN <= kHalfMaxMN ? HALF_SM : WHOLE_SM) - lz_bytes(MN) - BARS_BYTES - 1024u;
+  const int n = (int)(room / stage_bytes(MN));
+  return n < MAX_STAGES ? n : MAX_STAGES;
+}
+__host__ __device__ constexpr uint32_t smem_total(int MN) {
+  return (uint32_t)num_stages(MN) * stage_bytes(MN) + lz_bytes(MN) + BARS_BYTES + 1024u;
+}
+static_assert(2 * (smem_total(16) + 1024) <= 228 * 1024 && 2 * (smem_total(32) + 1024) <= 228 * 1024 &&
+                  2 * (smem_total(64) + 1024) <= 228 * 1024 && smem_total(128) <= 227 * 1024 && num_stages(64) >= 3,
+              "shared memory budget");
 
 struct Params {
   CUtensorMap w;     // W codes [N, K], box 128 rows x 128 bytes
@@ -49,6 +71,9 @@ struct Params {
   const float* bias;  // may be null
   int relu;
   int vec;           // rows of the output may be written 16 bytes at a time
+  float* amax;       // may be null: amax[m] = largest |Y[m, :]|
+  float* amax_part;  // with it: [tiles][MN] partial maxima, and the block ticket that finds the last CTA
+  uint32_t* ticket;
   uint32_t* status;
 };
 
@@ -96,7 +121,11 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i8_skinny_kernel(const __
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;  // same offset in every CTA of the cluster
-  const uint32_t bars = base + BARS_OFF;
+  const int MN = p.MN;
+  const int stages = num_stages(MN);
+  const uint32_t stride = stage_bytes(MN);
+  const uint32_t lz = base + (uint32_t)stages * stride;
+  const uint32_t bars = lz + lz_bytes(MN);
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (MAX_STAGES + s); };
   const uint32_t tfull_bar = bars + 8u * (2 * MAX_STAGES);
@@ -105,13 +134,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i8_skinny_kernel(const __
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = S > 1 ? cluster_ctarank() : 0u;
-  const uint32_t lz = base + RING_BYTES;
   const int tile = blockIdx.x / S;
   const int n0 = tile * BNCH;
-  const int MN = p.MN;
-  const uint32_t a_bytes = (uint32_t)MN * 128u;
-  const uint32_t stride = W_TILE + a_bytes;
-  const int stages = (int)(RING_BYTES / stride) < MAX_STAGES ? (int)(RING_BYTES / stride) : MAX_STAGES;
   const int total_kb = (p.K + 127) / 128;
   const int per = (total_kb + S - 1) / S;
   const int kb_begin = (int)rank * per;
@@ -140,7 +164,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i8_skinny_kernel(const __
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // launched early (programmatic stream serialisation): the set-up above overlapped the tail of the
-  // kernel in front; global memory is first touched after this wait
+  // kernel in front; global memory is first read after this wait.  The first ring of weights is on its way to L2
+  // before it (a prefetch moves no values: it does not matter whether the kernel in front writes them).
+  if (warp == 0 && lane < stages && kb_begin + lane < kb_end)
+    ptx::prefetch_tile_2d(&p.w, (kb_begin + lane) * 128, n0);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // "this CTA runs": waited for (by then for nothing) before the first store into a peer's memory
@@ -259,8 +286,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i8_skinny_kernel(const __
     const bool hb = p.bias != nullptr;
     auto finish = [&](int m, int4 s, float a) {
       const size_t off = (size_t)m * p.N + n;
+      float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
       if (FUSED) {
-        float4 y;
         y.x = dequant(s.x, a, w4.x, b4.x, hb, p.relu);
         y.y = dequant(s.y, a, w4.y, b4.y, hb, p.relu);
         y.z = dequant(s.z, a, w4.z, b4.z, hb, p.relu);
@@ -283,6 +310,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i8_skinny_kernel(const __
           if (n + 3 < p.N) p.acc[off + 3] = s.w;
         }
       }
+      if (FUSED && p.amax != nullptr) {  // this tile's part of the row maximum
+        float t = n < p.N ? fabsf(y.x) : 0.0f;
+        if (n + 1 < p.N) t = fmaxf(t, fabsf(y.y));
+        if (n + 2 < p.N) t = fmaxf(t, fabsf(y.z));
+        if (n + 3 < p.N) t = fmaxf(t, fabsf(y.w));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
+        if (lane == 0) p.amax_part[(size_t)tile * MN + m] = t;
+      }
     };
     const int rows_per = MN / S;
     int i = 0;
@@ -298,6 +334,18 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i8_skinny_kernel(const __
         s.x += t[r].x; s.y += t[r].y; s.z += t[r].z; s.w += t[r].w;
       }
       finish(m, s, __shfl_sync(0xffffffffu, sa_mine, i & 31));
+    }
+  }
+
+  // ------------------------------------------------------------ row maxima: the last CTA folds the tiles' parts
+  if (FUSED && p.amax != nullptr && vtlb_last_block(p.ticket)) {
+    const int tiles = (int)gridDim.x / S;
+    for (int m = warp; m < p.M; m += NUM_THREADS / 32) {
+      float t = 0.0f;
+      for (int i = lane; i < tiles; i += 32) t = fmaxf(t, __ldcg(p.amax_part + (size_t)i * MN + m));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
+      if (lane == 0) p.amax[m] = t;
     }
   }
 
@@ -318,19 +366,23 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_i8_skinny_kernel(const __
 // ---------------------------------------------------------------- host side
 constexpr int kMaxM = 128;
 
-// One wave of tiles: with more tiles than SMs the general kernel's wider tiles move fewer bytes.
+inline int row_class(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
+
+// Up to 64 rows any number of tiles (two CTAs share an SM); above, one wave of tiles: with more of them than
+// SMs the general kernel's wider tiles move fewer bytes.
 inline bool usable(vtlb_ctx* ctx, int M, int N) {
-  return M >= 1 && M <= kMaxM && N >= 1 && (N + BNCH - 1) / BNCH <= ctx->sm_count;
+  return M >= 1 && M <= kMaxM && N >= 1 && (M <= kHalfMaxMN || (N + BNCH - 1) / BNCH <= ctx->sm_count);
 }
 
 template <bool FUSED, int S>
-int configure(vtlb_ctx* ctx, int* max_clusters) {
+int configure(vtlb_ctx* ctx, int MN, int* max_clusters) {
   auto kern = gemm_i8_skinny_kernel<FUSED, S>;
-  VTLB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_TOTAL));
+  VTLB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_total(128)));
+  VTLB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(ctx->sm_count / S * S));
+  cfg.gridDim = dim3((unsigned)(2 * ctx->sm_count / S * S));
   cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = SMEM_TOTAL;
+  cfg.dynamicSmemBytes = smem_total(MN);
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)S;
@@ -347,7 +399,7 @@ int launch_s(vtlb_ctx* ctx, int tiles, const Params& p) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(tiles * S));
   cfg.blockDim = dim3(NUM_THREADS);
-  cfg.dynamicSmemBytes = SMEM_TOTAL;
+  cfg.dynamicSmemBytes = smem_total(p.MN);
   cfg.stream = ctx->stream;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -365,27 +417,36 @@ int launch_s(vtlb_ctx* ctx, int tiles, const Params& p) {
 // `p` arrives with the output pointers, scales, bias and relu filled in.
 template <bool FUSED>
 int launch(vtlb_ctx* ctx, const void* Aq, const void* Wq, int M, int N, int K, Params p) {
-  static int max_clusters[64][3];  // per device: clusters of 1, 2, 4 CTAs resident at a time
+  static int max_clusters[64][4][3];  // per device and row class: clusters of 1, 2, 4 CTAs resident at a time
   static std::atomic<uint64_t> configured{0};
   const int d = ctx->device & 63;
-  if (!(configured.load(std::memory_order_relaxed) >> d & 1)) {
-    int rc = configure<FUSED, 1>(ctx, &max_clusters[d][0]);
-    if (!rc) rc = configure<FUSED, 2>(ctx, &max_clusters[d][1]);
-    if (!rc) rc = configure<FUSED, 4>(ctx, &max_clusters[d][2]);
-    if (rc) return rc;
-    configured.fetch_or(1ull << d, std::memory_order_relaxed);
+  if (!(configured.load(std::memory_order_acquire) >> d & 1)) {
+    for (int i = 0; i < 4; ++i) {
+      int rc = configure<FUSED, 1>(ctx, 16 << i, &max_clusters[d][i][0]);
+      if (!rc) rc = configure<FUSED, 2>(ctx, 16 << i, &max_clusters[d][i][1]);
+      if (!rc) rc = configure<FUSED, 4>(ctx, 16 << i, &max_clusters[d][i][2]);
+      if (rc) return rc;
+    }
+    configured.fetch_or(1ull << d, std::memory_order_release);
   }
   const int ldk = (K + 15) / 16 * 16;
-  const int MN = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  const int MN = row_class(M);
+  const int* clusters = max_clusters[d][MN == 16 ? 0 : MN == 32 ? 1 : MN == 64 ? 2 : 3];
   const int tiles = (N + BNCH - 1) / BNCH;
   const int total_kb = (K + 127) / 128;
   // as many K ranges as still run in one wave (and leave every CTA at least two K blocks)
   int S = 1;
   for (int i = 2; i >= 1; --i)
-    if (tiles <= max_clusters[d][i] && total_kb >= 2 * (1 << i)) {
+    if (tiles <= clusters[i] && total_kb >= 2 * (1 << i)) {
       S = 1 << i;
       break;
     }
+  if (p.amax) {
+    void* part = nullptr;
+    if (int rc = vtlb_scratch(ctx, (size_t)tiles * MN * sizeof(float), &part)) return rc;
+    p.amax_part = (float*)part;
+    p.ticket = ctx->d_status + vtlb_ctx::kTicketWord;
+  }
   int rc = gemm::encode_tmap_2d(ctx, &p.w, false, Wq, (uint64_t)K, (uint64_t)N, (uint64_t)ldk, 128, BNCH);
   if (rc) return rc;
   rc = gemm::encode_tmap_2d(ctx, &p.a, false, Aq, (uint64_t)K, (uint64_t)M, (uint64_t)ldk, 128, (uint32_t)MN);

@@ -31,12 +31,15 @@ __device__ __forceinline__ int quant1(float a, float inv) {
 // re-reads the row (it is still in L1/L2: a row is at most a few tens of KB)
 // and writes 16 codes per thread as one 16-byte store.  Algorithmic HBM traffic:
 // 4K bytes read + K bytes written + 4 bytes of scale per row.
+// With the maxima given the values are independent, and a row is cut into gridDim.y pieces of `piece` values:
+// eight rows of 28672 on eight CTAs took 6.0 us, in 56 pieces 2.3 us.
+constexpr int kQuantPiece = 4096;  // 16 values a thread
 template <bool HAVE_AMAX>
 __global__ void __launch_bounds__(256) quant_rows_i8_kernel(const float* __restrict__ A, int M,
                                                             int K, int ldq,
                                                             int8_t* __restrict__ Q,
                                                             float* __restrict__ scale,
-                                                            const float* __restrict__ amax_in) {
+                                                            const float* __restrict__ amax_in, int piece) {
   __shared__ float s_part[8];
   __shared__ float s_amax;
   asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early: the kernel in front is done from here on
@@ -71,12 +74,14 @@ __global__ void __launch_bounds__(256) quant_rows_i8_kernel(const float* __restr
     amax = s_amax;
   }
   const float inv = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-  if (threadIdx.x == 0) scale[row] = __fdiv_rn(amax, 127.0f);
+  if (threadIdx.x == 0 && blockIdx.y == 0) scale[row] = __fdiv_rn(amax, 127.0f);
   int8_t* q = Q + (size_t)row * ldq;
+  const int k0 = HAVE_AMAX ? blockIdx.y * piece : 0;
+  const int k1 = HAVE_AMAX && K - k0 > piece ? k0 + piece : K;
   if (vec && (K & 15) == 0) {
     const float4* a4 = reinterpret_cast<const float4*>(a);
     int4* q16 = reinterpret_cast<int4*>(q);
-    for (int i = threadIdx.x; i < K / 16; i += blockDim.x) {
+    for (int i = k0 / 16 + threadIdx.x; i < k1 / 16; i += blockDim.x) {
       int w[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -88,7 +93,7 @@ __global__ void __launch_bounds__(256) quant_rows_i8_kernel(const float* __restr
       q16[i] = make_int4(w[0], w[1], w[2], w[3]);
     }
   } else {
-    for (int i = threadIdx.x; i < K; i += blockDim.x) q[i] = (int8_t)quant1(a[i], inv);
+    for (int i = k0 + threadIdx.x; i < k1; i += blockDim.x) q[i] = (int8_t)quant1(a[i], inv);
   }
 }
 
@@ -251,19 +256,24 @@ struct EpiDequant {
 // U * 512 bytes, all U 16-byte loads of a lane issued before the first is used (a whole
 // 4096-byte row in flight per warp at U = 8), accumulating with dp4a against up to MT
 // rows of A (exact int32).
-template <int MT, int U, bool FUSED>
+template <int MT, int U, bool FUSED, bool AMAX>
 __global__ void __launch_bounds__(128) gemv_i8_kernel(const int8_t* __restrict__ Aq,
                                                       const int8_t* __restrict__ Wq, int M, int N,
                                                       int K, int ldk, int32_t* __restrict__ acc_out,
                                                       float* __restrict__ Y,
                                                       const float* __restrict__ sa,
                                                       const float* __restrict__ sw,
-                                                      const float* __restrict__ bias, int relu) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early: the kernel in front is done from here on
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+                                                      const float* __restrict__ bias, int relu,
+                                                      float* __restrict__ amax,  // AMAX: amax[m] = max |Y[m, :]|
+                                                      float* __restrict__ amax_part, uint32_t* ticket) {
   const int lane = threadIdx.x & 31;
   const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early: the kernel in front is done from here on
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  float ymax[MT];  // lane 0: largest |y| of the channels this warp has finished
+#pragma unroll
+  for (int m = 0; m < MT; ++m) ymax[m] = 0.0f;
   for (int n = gwarp; n < N; n += nwarps) {
     int acc[MT];
 #pragma unroll
@@ -316,13 +326,34 @@ __global__ void __launch_bounds__(128) gemv_i8_kernel(const int8_t* __restrict__
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
         if (m >= M) continue;
-        if (FUSED)
-          Y[(size_t)m * N + n] = dequant1((uint32_t)acc[m], sa[m], sw[n], bias ? bias[n] : 0.0f,
-                                          bias != nullptr, relu);
-        else
+        if (FUSED) {
+          const float y = dequant1((uint32_t)acc[m], sa[m], sw[n], bias ? bias[n] : 0.0f, bias != nullptr, relu);
+          Y[(size_t)m * N + n] = y;
+          if (AMAX) ymax[m] = fmaxf(ymax[m], fabsf(y));
+        } else {
           acc_out[(size_t)m * N + n] = acc[m];
+        }
       }
     }
+  }
+  if (!AMAX) return;
+  // row maxima: every CTA leaves one value per row, the last CTA folds them
+  __shared__ float s_max[4][MT];
+  const int warp = threadIdx.x >> 5;
+  if (lane == 0) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m) s_max[warp][m] = ymax[m];
+  }
+  __syncthreads();
+  if (threadIdx.x < MT && (int)threadIdx.x < M)
+    amax_part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] =
+        fmaxf(fmaxf(s_max[0][threadIdx.x], s_max[1][threadIdx.x]), fmaxf(s_max[2][threadIdx.x], s_max[3][threadIdx.x]));
+  if (!vtlb_last_block(ticket)) return;
+  for (int m = warp; m < M; m += 4) {
+    float t = 0.0f;
+    for (int i = lane; i < (int)gridDim.x; i += 32) t = fmaxf(t, __ldcg(amax_part + (size_t)m * gridDim.x + i));
+    t = warp_max(t);
+    if (lane == 0) amax[m] = t;
   }
 }
 
@@ -353,14 +384,19 @@ bool use_skinny(vtlb_ctx* ctx, int M, int N) {
 template <bool FUSED>
 int launch_gemv(vtlb_ctx* ctx, const int8_t* Aq, const int8_t* Wq, int M, int N, int K,
                 int32_t* acc, float* Y, const float* sa, const float* sw, const float* bias,
-                int relu) {
+                int relu, float* amax = nullptr) {
   const int ldk = vtlb_i8_ld(K);
   int blocks = (N + 3) / 4;  // four warps per block, one channel per warp at a time
   if (blocks > ctx->sm_count * 8) blocks = ctx->sm_count * 8;
   if (blocks < 1) blocks = 1;
+  void* part = nullptr;
+  if (amax)
+    if (int rc = vtlb_scratch(ctx, (size_t)blocks * M * sizeof(float), &part)) return rc;
 #define VTLB_GEMV(MT)                                                                        \
-  VTLB_CUDA(ctx, vtlb_launch_early(gemv_i8_kernel<MT, 8, FUSED>, dim3(blocks), dim3(128), 0, ctx->stream, \
-                                   Aq, Wq, M, N, K, ldk, acc, Y, sa, sw, bias, relu))
+  VTLB_CUDA(ctx, vtlb_launch_early(amax ? gemv_i8_kernel<MT, 8, FUSED, FUSED> : gemv_i8_kernel<MT, 8, FUSED, false>, \
+                                   dim3(blocks), dim3(128), 0, ctx->stream,                  \
+                                   Aq, Wq, M, N, K, ldk, acc, Y, sa, sw, bias, relu, amax, (float*)part, \
+                                   ctx->d_status + vtlb_ctx::kTicketWord))
   if (M <= 1) VTLB_GEMV(1);
   else if (M <= 2) VTLB_GEMV(2);
   else if (M <= 4) VTLB_GEMV(4);
@@ -489,13 +525,15 @@ VTLB_API int vtlb_quant_rows_i8(vtlb_ctx* ctx, const void* d_A, int M, int K, vo
     VTLB_LAUNCHED(ctx);
     return VTLB_OK;
   }
-  if (d_amax_in_or_null)
-    quant_rows_i8_kernel<true><<<M, 256, 0, ctx->stream>>>((const float*)d_A, M, K, ldq,
-                                                           (int8_t*)d_Q, (float*)d_scale,
-                                                           (const float*)d_amax_in_or_null);
+  const int piece = K <= kQuantPiece * 65535ll ? kQuantPiece : 16 * kQuantPiece;  // gridDim.y is at most 65535
+  const dim3 grid(M, d_amax_in_or_null ? (unsigned)(((long long)K + piece - 1) / piece) : 1u);
+  auto kern = d_amax_in_or_null ? quant_rows_i8_kernel<true> : quant_rows_i8_kernel<false>;
+  if (M > kEarlyQuantRows)
+    kern<<<grid, 256, 0, ctx->stream>>>((const float*)d_A, M, K, ldq, (int8_t*)d_Q, (float*)d_scale,
+                                        (const float*)d_amax_in_or_null, piece);
   else
-    quant_rows_i8_kernel<false><<<M, 256, 0, ctx->stream>>>((const float*)d_A, M, K, ldq,
-                                                            (int8_t*)d_Q, (float*)d_scale, nullptr);
+    VTLB_CUDA(ctx, vtlb_launch_early(kern, grid, dim3(256), 0, ctx->stream, (const float*)d_A, M, K, ldq, (int8_t*)d_Q,
+                                     (float*)d_scale, (const float*)d_amax_in_or_null, piece));
   VTLB_LAUNCHED(ctx);
   return VTLB_OK;
 }
@@ -547,7 +585,8 @@ static int linear_i8_fwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_Aq, i
   if (shards == 1 && (M <= gemv_max_m() || use_skinny(ctx, M, N))) {
     if (M <= gemv_max_m()) {
       rc = launch_gemv<true>(ctx, (const int8_t*)d_Aq, (const int8_t*)d_Wq, M, N, K, nullptr, (float*)d_Y,
-                             (const float*)d_sa, (const float*)d_sw, (const float*)d_bias_or_null, relu);
+                             (const float*)d_sa, (const float*)d_sw, (const float*)d_bias_or_null, relu,
+                             (float*)d_row_amax_or_null);
     } else {
       skinny::Params p = {};
       p.Y = (float*)d_Y;
@@ -555,12 +594,10 @@ static int linear_i8_fwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_Aq, i
       p.sw = (const float*)d_sw;
       p.bias = (const float*)d_bias_or_null;
       p.relu = relu;
+      p.amax = (float*)d_row_amax_or_null;
       rc = skinny::launch<true>(ctx, d_Aq, d_Wq, M, N, K, p);
     }
-    if (rc || !d_row_amax_or_null) return rc;
-    row_absmax_kernel<<<M, 256, 0, ctx->stream>>>((const float*)d_Y, M, N, (float*)d_row_amax_or_null);
-    VTLB_LAUNCHED(ctx);
-    return VTLB_OK;
+    return rc;
   }
   EpiDequant epi{(float*)d_Y, (const float*)d_sa, (const float*)d_sw, (const float*)d_bias_or_null, N, relu};
   if (d_row_amax_or_null) {
