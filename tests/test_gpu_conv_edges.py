@@ -1,0 +1,50 @@
+"""Convolution against 64-bit sums (torch on the CPU) where its kernels change over."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(terms, a, b):
+    # three TF32 products per f32 product leave 2^-21 of each term, sums of `terms` of them round to f32
+    return 1e-5 * np.sqrt(terms) * float(np.abs(a).max()) * float(np.abs(b).max())
+
+
+def _check(dev, B, C, H, W, O, k, pad, stride, relu=True, bias=True):
+    rng = np.random.default_rng(B + 10 * C + 100 * H + O + k)
+    x = rng.standard_normal((B, C, H, W)).astype(np.float32)
+    w = (rng.standard_normal((O, C, k, k)) * (2.0 / (C * k * k)) ** 0.5).astype(np.float32)
+    b = rng.standard_normal(O).astype(np.float32) if bias else None
+    t = lambda a: torch.from_numpy(a).double()  # noqa: E731
+    pre = torch.nn.functional.conv2d(t(x), t(w), t(b) if bias else None, stride, pad).numpy()
+    OH, OW = pre.shape[2:]
+    g = rng.standard_normal(pre.shape).astype(np.float32)
+    rdx = torch.nn.grad.conv2d_input(x.shape, t(w), t(g), stride, pad).numpy()
+    rdw = torch.nn.grad.conv2d_weight(t(x), w.shape, t(g), stride, pad).numpy()
+    rdb = g.astype(np.float64).sum(axis=(0, 2, 3))
+    d = [dev.to_device(a) for a in (x, w, g)]
+    db_in = dev.to_device(b) if bias else None
+    out = [dev.to_device(np.full(s, np.nan, np.float32)) for s in (pre.shape, pre.shape, x.shape, w.shape, (O,))]
+    dims = (B, C, H, W, O, k, k, pad, pad, stride, stride)
+    dev.conv2d_fwd_f32(d[0], d[1], db_in, out[0], *dims, relu, out[1])
+    dev.conv2d_bwd_f32(d[2], d[0], d[1], out[2], out[3], out[4], *dims)
+    assert dev.check_status() == 0
+    y, p, dx, dw, db = (o.numpy() for o in out)
+    fwd = _bound(C * k * k, x, w) + (2e-7 * np.abs(b).max() if bias else 0)
+    assert np.abs(p - pre).max() <= fwd
+    assert np.array_equal(y, np.where(p < 0, np.float32(0), p) if relu else p)
+    assert np.abs(dx - rdx).max() <= _bound(O * k * k, g, w)
+    assert np.abs(dw - rdw).max() <= _bound(B * OH * OW, g, x)
+    assert np.abs(db - rdb).max() <= 1e-6 * max(1.0, np.abs(g).sum(axis=(0, 2, 3)).max())
+    for o in d + out + ([db_in] if bias else []):
+        o.free()
+
+
+@pytest.mark.parametrize("B,C,H,W,O,k,pad,stride", [
+    (2, 3, 11, 14, 5, 3, 0, 2), (3, 4, 12, 9, 6, 3, 1, 2), (1, 2, 7, 7, 3, 3, 2, 2),   # window rows and columns left over
+    (2, 5, 15, 16, 4, 5, 2, 2), (1, 1, 5, 5, 2, 5, 0, 2), (2, 3, 13, 40, 9, 5, 1, 2),
+    (2, 3, 10, 11, 4, 4, 1, 2), (2, 3, 11, 10, 4, 3, 1, 3), (2, 6, 9, 9, 7, 1, 0, 2),  # any window, any stride
+])
+def test_strided_windows(dev, B, C, H, W, O, k, pad, stride):
+    _check(dev, B, C, H, W, O, k, pad, stride)
