@@ -1,0 +1,104 @@
+"""f32 products large enough for the CTA-pair kernel on f16 planes, against 64-bit products; and operands that f16
+planes cannot hold, which have to come out as well as 3xTF32 does."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _error(C, A, B):
+    """Largest error of C against A @ B^T, over |A| @ |B|^T element by element."""
+    A, B = torch.from_numpy(A).double().cuda(), torch.from_numpy(B).double().cuda()
+    d = (torch.from_numpy(C).double().cuda() - A @ B.T).abs()
+    return float((d / (A.abs() @ B.abs().T).clamp_min(1e-300)).max())
+
+
+# Operands keep 22 bits (2^-22 a factor, twice); an accumulator of tcgen05 truncates, at most 24 times before it is
+# closed (8 K steps x 3 products), by less than 2^-23 of the sum of magnitudes each; the closed ones round to nearest.
+BOUND = 2 * 2.0**-22 + 24 * 2.0**-23
+
+
+def _product(dev, ta, tb, A, B):
+    M, K = A.shape
+    N = B.shape[0]
+    dA = dev.to_device(np.ascontiguousarray(A.T if ta else A))
+    dB = dev.to_device(np.ascontiguousarray(B if tb else B.T))
+    dC = dev.to_device(np.full((M, N), np.nan, np.float32))
+    dev.gemm_f32(ta, tb, M, N, K, dA, dB, dC)
+    assert dev.check_status() == 0
+    C = dC.numpy()
+    for b in (dA, dB, dC):
+        b.free()
+    return C
+
+
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(2048, 1280, 63), (1500, 1800, 255), (1537, 1793, 256), (2049, 1279, 257),
+                                   (512, 4868, 1001), (2500, 1003, 516)])
+def test_product(dev, ta, tb, M, N, K):
+    rng = np.random.default_rng(M + N + K)
+    A, B = (rng.standard_normal((r, K)).astype(np.float32) for r in (M, N))
+    assert _error(_product(dev, ta, tb, A, B), A, B) < BOUND
+
+
+def _features(rng, r, K, sign):
+    return rng.standard_normal((r, K)) * 10.0 ** (sign * 12 * (np.arange(K) % 7 / 6 - 0.5))
+
+
+@pytest.mark.parametrize("kind", ["features", "rows", "tiny", "huge", "lognormal", "zeros", "sparse"])
+def test_operands_of_any_range(dev, kind):
+    M, N, K = 1536, 1792, 600
+    rng = np.random.default_rng(3)
+    A, B = rng.standard_normal((M, K)), rng.standard_normal((N, K))
+    if kind == "features":  # columns on scales 1e-6 .. 1e6, undone by the weights
+        A, B = _features(rng, M, K, 1), _features(rng, N, K, -1)
+    if kind == "rows":      # every output on a scale of its own, both sides
+        A, B = A * 10.0 ** rng.uniform(-8, 8, (M, 1)), B * 10.0 ** rng.uniform(-8, 8, (N, 1))
+    if kind == "tiny":
+        A, B = A * 1e-25, B * 1e-8
+    if kind == "huge":
+        A, B = A * 1e30, B * 1e-20
+    if kind == "lognormal":
+        A, B = A * np.exp(3 * rng.standard_normal(A.shape)), B * np.exp(3 * rng.standard_normal(B.shape))
+    if kind == "zeros":
+        A[:, 256:512], B[100:200] = 0, 0
+    if kind == "sparse":    # a few values a row, on scales of their own
+        A = A * (rng.random(A.shape) < 0.01) * 10.0 ** rng.uniform(-9, 0, A.shape)
+    A, B = A.astype(np.float32), B.astype(np.float32)
+    # 3xTF32 closes an accumulator after 48 products; the operands keep the same 22 bits
+    assert _error(_product(dev, False, True, A, B), A, B) < 2 * 2.0**-22 + 48 * 2.0**-23
+
+
+def test_infinities_and_nans_stay_in_their_rows(dev):
+    M, N, K = 1536, 1792, 512
+    rng = np.random.default_rng(4)
+    A, B = (rng.standard_normal((r, K)).astype(np.float32) for r in (M, N))
+    A[3, 300], A[700, 0], B[9, 511] = np.inf, np.nan, -np.inf
+    C = _product(dev, False, True, A, B)
+    assert not np.isfinite(C[3]).any() and np.isnan(C[700]).all() and not np.isfinite(C[:, 9]).any()
+    rows, cols = np.delete(np.arange(M), [3, 700]), np.delete(np.arange(N), 9)
+    assert _error(np.ascontiguousarray(C[rows][:, cols]), A[rows], B[cols]) < 2 * 2.0**-22 + 48 * 2.0**-23
+
+
+@pytest.mark.parametrize("wide", [False, True])
+def test_linear_backward(dev, wide):
+    """dX masked by the layer below, dW, and the bias gradient that the transposing pass sums on the way."""
+    M, N, K = 1300, 1600, 1540
+    rng = np.random.default_rng(5)
+    g, x, w, mask = (rng.standard_normal(s).astype(np.float32) for s in ((M, N), (M, K), (N, K), (M, K)))
+    if wide:  # unfit for f16 planes: the bias gradient still comes from their pass
+        g = (g * 10.0 ** rng.uniform(-9, 0, g.shape)).astype(np.float32)
+    d = [dev.to_device(a) for a in (g, x, w, mask)]
+    out = [dev.to_device(np.full(s, np.nan, np.float32)) for s in ((M, K), (N, K), (N,))]
+    dev.linear_bwd_f32_planes(d[0], d[1], d[2], out[0], out[1], out[2], M, N, K, relu_mask_src=d[3])
+    assert dev.check_status() == 0
+    dx, dw, db = (o.numpy() for o in out)
+    assert (dx[mask < 0] == 0).all()
+    full = np.where(mask < 0, (g.astype(np.float64) @ w.astype(np.float64)).astype(np.float32), dx)
+    assert _error(full, g, np.ascontiguousarray(w.T)) < 2 * 2.0**-22 + 48 * 2.0**-23
+    assert _error(dw, np.ascontiguousarray(g.T), np.ascontiguousarray(x.T)) < 2 * 2.0**-22 + 48 * 2.0**-23
+    ref = g.astype(np.float64).sum(axis=0)
+    assert (np.abs(db - ref) <= 2.0**-24 * np.abs(ref) + 1e-13 * np.abs(g).sum(axis=0)).all()
+    for b in d + out:
+        b.free()

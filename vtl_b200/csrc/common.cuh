@@ -31,8 +31,11 @@ struct vtlb_ctx {
   // next batch comes in and the last result goes out while the current step computes
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
   cudaEvent_t ev_copy = nullptr;       // ordering between the copy streams and compute
-  uint32_t* d_status = nullptr;        // device status word, and (kTicketWord) the block ticket of last_block()
-  static constexpr int kTicketWord = 32;
+  // device status word, (kTicketWord) the block ticket of last_block() and (kUnfitWord) the epoch of the last
+  // f32 product whose operands did not fit f16 planes
+  uint32_t* d_status = nullptr;
+  static constexpr int kTicketWord = 32, kUnfitWord = 40;
+  uint32_t half_epoch = 0;             // products on f16 planes so far, never 0
   void* scratch = nullptr;             // operand-split buffers, partial sums
   size_t scratch_bytes = 0;
   // INT8 pair GEMM, K-split tiles: flags + parked accumulators (kKsplitBytes, allocated with the

@@ -78,6 +78,212 @@ __global__ void __launch_bounds__(256) split_transpose_kernel(const float* __res
   }
 }
 
+// The multiplier 2^e that brings a block's largest magnitude into [2^14, 2^15), and 2^-e.  e is kept where both
+// are normal numbers; a block of zeros (or of NaNs) gets 1.
+__device__ __forceinline__ void block_scale(float amax, float& mul, float& inv) {
+  const int ex = (int)(__float_as_uint(amax) >> 23);  // biased exponent; 255 for an infinity
+  const int e = amax > 0.0f ? min(126, 14 + 127 - ex) : 0;
+  mul = __uint_as_float((uint32_t)(127 + e) << 23);
+  inv = __uint_as_float((uint32_t)(127 - e) << 23);
+}
+__device__ __forceinline__ void split_half(float x, __half& hi, __half& lo) {
+  hi = __float2half_rn(x);
+  lo = __float2half_rn(x - __half2float(hi));
+}
+__device__ __forceinline__ float warp_amax(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+// Largest of the eight warps' values; everybody gets it.
+__device__ __forceinline__ float block_amax(float v, float (&part)[8]) {
+  v = warp_amax(v);
+  __syncthreads();  // the previous use of part is over
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = part[0];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) v = fmaxf(v, part[w]);
+  return v;
+}
+// Says that f16 cannot hold a block of 256 values, eight per lane, as well as TF32 does (struct HalfPlanes): more
+// than one in sixteen of those that are not zero (and more than a stray one) scaled below 2^-4, or a scale so
+// extreme that the product of two such would leave the f32 range (an infinity in the block among them).
+__device__ __forceinline__ void note_unfit(const float (&v)[8], float mul, uint32_t* unfit, uint32_t epoch) {
+  uint32_t n = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float a = fabsf(v[j]);
+    n += (a > 0.0f ? 1u : 0u) + (a > 0.0f && a * mul < 0.0625f ? 0x10000u : 0u);
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  const uint32_t small = n >> 16, nonzero = n & 0xffffu;
+  const bool extreme = mul > 1.8889466e22f || mul < 1.0842022e-19f;  // 2^74, 2^-63
+  if ((threadIdx.x & 31) == 0 && (extreme || (small >= 2 && small * 16 > nonzero))) *unfit = epoch;
+}
+
+// src [R, C] row-major -> scaled f16 planes [R, ld] and factors.  A CTA takes 32 rows x 256 values, a warp four of
+// the rows, eight values per lane.  GROUP: one scale for the 32 rows (operand B), else one per row.
+// Bound by HBM, 8 bytes per element: 8192 x 4096 in 43 us (6.2 TB/s); the TF32 planes, 12 bytes, took 70 us.
+template <bool VEC, bool GROUP>
+__global__ void __launch_bounds__(256) split_rows_half_kernel(const float* __restrict__ src, int R, int C, int ld,
+                                                              int lds, __half* __restrict__ hi,
+                                                              __half* __restrict__ lo, float* __restrict__ scale,
+                                                              uint32_t* unfit, uint32_t epoch) {
+  __shared__ float part[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int blocks = (C + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
+  const long long n = (long long)((R + 31) / 32) * blocks;
+  for (long long t = blockIdx.x; t < n; t += gridDim.x) {
+    const int grp = (int)(t / blocks), kb = (int)(t - (long long)grp * blocks);
+    const int c = kb * gemm::kHalfBlock + lane * 8, r0 = grp * 32 + warp * 4;
+    float v[4][8], m[4], all = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float* a = src + (size_t)(r0 + q) * C + c;
+      const bool row = r0 + q < R;
+      if (VEC) {
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 u0 = row && c < C ? __ldg(reinterpret_cast<const float4*>(a)) : z;  // C % 4 == 0
+        const float4 u1 = row && c + 4 < C ? __ldg(reinterpret_cast<const float4*>(a) + 1) : z;
+        v[q][0] = u0.x; v[q][1] = u0.y; v[q][2] = u0.z; v[q][3] = u0.w;
+        v[q][4] = u1.x; v[q][5] = u1.y; v[q][6] = u1.z; v[q][7] = u1.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[q][j] = row && c + j < C ? __ldg(a + j) : 0.0f;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      m[q] = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) m[q] = fmaxf(m[q], fabsf(v[q][j]));
+      all = fmaxf(all, m[q]);
+    }
+    if (GROUP) all = block_amax(all, part);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float mul, inv;
+      block_scale(GROUP ? all : warp_amax(m[q]), mul, inv);
+      note_unfit(v[q], mul, unfit, epoch);
+      if (r0 + q >= R) break;
+      union { __half h[8]; uint4 u; } ph, pl;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) split_half(v[q][j] * mul, ph.h[j], pl.h[j]);
+      if (c < ld) {  // ld is C rounded up to 8
+        *reinterpret_cast<uint4*>(hi + (size_t)(r0 + q) * ld + c) = ph.u;
+        *reinterpret_cast<uint4*>(lo + (size_t)(r0 + q) * ld + c) = pl.u;
+      }
+      if (!GROUP && lane == 0) scale[(size_t)kb * lds + r0 + q] = inv;
+      if (GROUP && threadIdx.x == 0 && q == 0) scale[(size_t)kb * lds + grp] = inv;
+    }
+  }
+}
+
+// src [R, C] row-major -> planes of the transpose, [C, ld >= R], and factors; where `colsum` is given, also the f64
+// column sums of each block, colsum[block][C] (the bias gradient's partial sums: a pass of its own over the gradient
+// took 71 us per 8192 x 4096).  A CTA turns 256 rows x 32 columns through shared memory: 128-byte rows in, and a
+// warp writes 128 contiguous bytes of a plane per instruction.  8192 x 4096: 57 us (73 us for TF32 planes).
+template <bool GROUP>
+__global__ void __launch_bounds__(256) split_transpose_half_kernel(const float* __restrict__ src, int R, int C, int ld,
+                                                                   int lds, __half* __restrict__ hi,
+                                                                   __half* __restrict__ lo, float* __restrict__ scale,
+                                                                   double* __restrict__ colsum, uint32_t* unfit,
+                                                                   uint32_t epoch) {
+  __shared__ float tile[gemm::kHalfBlock][33];
+  __shared__ float part[8];
+  const int tiles_c = (C + 31) / 32, tiles_r = (R + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
+  const long long ntiles = (long long)tiles_c * tiles_r;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int kb = (int)(t / tiles_c), r0 = kb * gemm::kHalfBlock, c0 = (int)(t - (long long)kb * tiles_c) * 32;
+    const int c = c0 + lane;
+    float all = 0.0f;
+    __syncthreads();  // the previous tile has been read
+#pragma unroll 16
+    for (int j = 0; j < gemm::kHalfBlock; j += 8) {
+      const int r = r0 + warp + j;
+      const float x = (r < R && c < C) ? __ldg(src + (size_t)r * C + c) : 0.0f;
+      tile[warp + j][lane] = x;
+      if (GROUP) all = fmaxf(all, fabsf(x));
+    }
+    if (GROUP) all = block_amax(all, part);
+    else __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int col = warp * 4 + q, cg = c0 + col;
+      if (cg >= C) break;
+      float v[8];
+      float m = 0.0f, mul, inv;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // rows i * 64 + lane * 2 + {0, 1}
+        v[2 * i] = tile[i * 64 + lane * 2][col];
+        v[2 * i + 1] = tile[i * 64 + lane * 2 + 1][col];
+        m = fmaxf(m, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
+      }
+      block_scale(GROUP ? all : warp_amax(m), mul, inv);
+      note_unfit(v, mul, unfit, epoch);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + i * 64 + lane * 2;
+        if (r < ld) {  // ld is R rounded up to 8
+          __half2 h, l;
+          split_half(v[2 * i] * mul, h.x, l.x);
+          split_half(v[2 * i + 1] * mul, h.y, l.y);
+          *reinterpret_cast<__half2*>(hi + (size_t)cg * ld + r) = h;
+          *reinterpret_cast<__half2*>(lo + (size_t)cg * ld + r) = l;
+        }
+      }
+      if (!GROUP && lane == 0) scale[(size_t)kb * lds + cg] = inv;
+      if (GROUP && threadIdx.x == 0 && q == 0) scale[(size_t)kb * lds + c0 / 32] = inv;
+      if (colsum) {
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s = __dadd_rn(s, (double)v[i]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        if (lane == 0) colsum[(size_t)kb * C + cg] = s;
+      }
+    }
+  }
+}
+
+// TF32 planes of both operands of a product whose operands do not fit f16 planes; returns at once for all others.
+struct SplitSource {
+  const float* src;
+  float *hi, *lo;
+  int rows, kdim, ld, transposed;  // transposed: stored [kdim, rows]
+};
+__global__ void __launch_bounds__(256) split_unfit_kernel(SplitSource a, SplitSource b, const uint32_t* unfit,
+                                                          uint32_t epoch) {
+  __shared__ float tile[32][33];
+  if (*unfit != epoch) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int o = 0; o < 2; ++o) {
+    const SplitSource s = o ? b : a;
+    const int tiles_k = (s.kdim + 31) / 32;
+    const long long ntiles = (long long)((s.rows + 31) / 32) * tiles_k;
+    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+      const int r0 = (int)(t / tiles_k) * 32, k0 = (int)(t % tiles_k) * 32;
+      if (s.transposed) {
+        __syncthreads();
+        for (int j = ty; j < 32; j += 8)
+          tile[j][tx] = k0 + j < s.kdim && r0 + tx < s.rows ? s.src[(size_t)(k0 + j) * s.rows + r0 + tx] : 0.0f;
+        __syncthreads();
+      }
+      for (int j = ty; j < 32; j += 8) {
+        const int r = r0 + j, k = k0 + tx;
+        if (r < s.rows && k < s.kdim) {
+          float h, l;
+          split1(s.transposed ? tile[tx][j] : s.src[(size_t)r * s.kdim + k], h, l);
+          s.hi[(size_t)r * s.ld + k] = h;
+          s.lo[(size_t)r * s.ld + k] = l;
+        }
+      }
+    }
+  }
+}
+
 // Column sums of G[M,N] in f64: partial[s][n] = sum over rows r == s (mod S).
 __global__ void __launch_bounds__(128) colsum_partial_kernel(const float* __restrict__ G, int M,
                                                              int N, double* __restrict__ partial) {
@@ -186,7 +392,31 @@ struct GemmExtras {
   const float* mask = nullptr;
   const vtlb_planes* out_rows = nullptr;
   const vtlb_planes* out_cols = nullptr;
+  // column sums of A as stored ([K, M], transA): the bias gradient, from the pass that transposes A; *colsum_done
+  // says whether that pass ran
+  float* a_colsum = nullptr;
+  bool* colsum_done = nullptr;
 };
+
+// Splits one operand into f16 planes; `transposed` says src is stored [kdim, rows], `group` that 32 rows share a
+// scale (operand B).
+int split_operand_half(vtlb_ctx* ctx, const float* src, int rows, int kdim, bool transposed, bool group, int ld, int lds,
+                       __half* hi, __half* lo, float* scale, double* colsum, uint32_t epoch) {
+  vtlb_prof_scope prof(ctx, VTLB_PHASE_SPLIT);
+  uint32_t* unfit = ctx->d_status + vtlb_ctx::kUnfitWord;
+  const int grid = f32::grid_for(ctx, (size_t)((rows + 31) / 32) * ((kdim + gemm::kHalfBlock - 1) / gemm::kHalfBlock), 1);
+  if (transposed) {
+    auto kern = group ? split_transpose_half_kernel<true> : split_transpose_half_kernel<false>;
+    kern<<<grid, 256, 0, ctx->stream>>>(src, kdim, rows, ld, lds, hi, lo, scale, colsum, unfit, epoch);
+  } else {
+    const bool vec = (kdim & 3) == 0 && vtlb_aligned16(src);
+    auto kern = group ? (vec ? split_rows_half_kernel<true, true> : split_rows_half_kernel<false, true>)
+                      : (vec ? split_rows_half_kernel<true, false> : split_rows_half_kernel<false, false>);
+    kern<<<grid, 256, 0, ctx->stream>>>(src, rows, kdim, ld, lds, hi, lo, scale, unfit, epoch);
+  }
+  VTLB_LAUNCHED(ctx);
+  return VTLB_OK;
+}
 
 int relu_mask_inplace(vtlb_ctx* ctx, float* C, const float* mask, size_t n) {
   return vtlb_relu_bwd_f32(ctx, C, mask, C, n);
@@ -199,7 +429,38 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
     return vtlb_fail(ctx, VTLB_EINVAL, "f32 GEMM: output and bias pointers must be 16-byte aligned");
   const int ld_rows = vtlb_plane_ld(N), ld_cols = vtlb_plane_ld(M);
   int rc, fused = 0;
-  if (2.0 * M * N * K <= ctx->small_gemm_flops) {  // launch-latency-bound sizes: CUDA cores, no split passes
+  const bool planes_in_or_out = ex.a_planes || ex.b_planes || ex.out_rows || ex.out_cols;
+  if (2.0 * M * N * K > ctx->small_gemm_flops && !planes_in_or_out && gemm2::pair_worthwhile(ctx, M, N)) {
+    // Large products: f16 planes on CTA pairs, twice the tensor rate of TF32 planes and half their bytes.  Planes
+    // that come in or go out are TF32 ones, so products with those keep the 3xTF32 kernel.
+    const int blocks = (K + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
+    const bool sums = ex.a_colsum && transA;
+    f32::HalfPlanes p;
+    if ((rc = f32::alloc_half_planes(ctx, M, N, K, sums ? (size_t)blocks * M * sizeof(double) + 256 : 0, &p))) return rc;
+    double* partial = sums ? (double*)vtlb_round_up((size_t)p.extra, 256) : nullptr;
+    if (++ctx->half_epoch == 0) ctx->half_epoch = 1;
+    const uint32_t epoch = ctx->half_epoch;
+    if ((rc = split_operand_half(ctx, A, M, K, transA != 0, false, p.ld, p.lda_scale, p.a_hi, p.a_lo, p.a_scale, partial,
+                                 epoch)))
+      return rc;
+    if ((rc = split_operand_half(ctx, B, N, K, transB == 0, true, p.ld, p.ldb_scale, p.b_hi, p.b_lo, p.b_scale, nullptr,
+                                 epoch)))
+      return rc;
+    if (sums) {
+      colsum_final_kernel<<<(M + 127) / 128, 128, 0, ctx->stream>>>(partial, blocks, M, ex.a_colsum);
+      VTLB_LAUNCHED(ctx);
+      *ex.colsum_done = true;
+    }
+    {
+      const SplitSource sa{A, p.tf32.a_hi, p.tf32.a_lo, M, K, p.tf32.ld, transA != 0};
+      const SplitSource sb{B, p.tf32.b_hi, p.tf32.b_lo, N, K, p.tf32.ld, transB == 0};
+      split_unfit_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(sa, sb, ctx->d_status + vtlb_ctx::kUnfitWord, epoch);
+      VTLB_LAUNCHED(ctx);
+    }
+    f32::EpiBiasRelu epi{C, bias, pre, N, relu};
+    epi.mask = ex.mask;
+    if ((rc = f32::launch_f16x3(ctx, p, M, N, K, epi, epoch, &fused))) return rc;
+  } else if (2.0 * M * N * K <= ctx->small_gemm_flops) {  // launch-latency-bound sizes: CUDA cores, no split passes
     if ((rc = f32::sgemm_small(ctx, transA, transB, M, N, K, A, B, C, bias, relu, pre, nullptr, nullptr, ex.mask)))
       return rc;
     if (ex.mask) fused |= 2;  // the mask is part of that kernel's epilogue
@@ -378,6 +639,8 @@ int linear_bwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_G, const void* 
       GemmExtras ex;
       ex.a_planes = g_cols;
       ex.b_planes = x_cols;
+      ex.a_colsum = (float*)d_db_or_null;
+      ex.colsum_done = &db_done;
       if ((rc = gemm_f32_impl(ctx, 1, 0, N, K, M, (const float*)d_G, (const float*)d_X, (float*)d_dW_or_null,
                               nullptr, 0, nullptr, ex)))
         return rc;

@@ -1,6 +1,7 @@
 // Pieces shared by the f32 GEMM users (f32.cu, conv.cu): the TF32 hi/lo split, the
 // operand planes in the context scratch, and the launcher of the 3xTF32 tcgen05 GEMM.
 #pragma once
+#include <cuda_fp16.h>
 #include <stdlib.h>
 
 #include "gemm_tc2.cuh"
@@ -46,6 +47,43 @@ inline int alloc_planes(vtlb_ctx* ctx, int rows_a, int rows_b, int K, size_t ext
   return VTLB_OK;
 }
 
+// Two K-major operands, each as a pair of f16 planes [rows, ld] of scaled values: a block of 256 elements along K
+// of a row of A (of 32 rows of B) is multiplied by the power of two that brings its largest into [2^14, 2^15), and
+//     x * 2^e = hi + lo,  hi = f16(x * 2^e), lo = f16(x * 2^e - hi).
+// hi and lo have 11 significant bits each, as TF32 has, so the three products lo.hi + hi.lo + hi.hi lose what the
+// 3xTF32 ones lose, 2^-22 of a term.  Where lo is below f16's normal range, an element keeps 2^-25 of its scaled
+// value instead: that is as good down to 2^-4 = 2^-18 of its block's largest.  The split passes count the elements
+// below that; a block with more than one in sixteen of them (features on very different scales, say) makes the
+// operands unfit, and the product runs on TF32 planes after all, from a launch behind this one that otherwise
+// returns at once.  The TF32 planes take the f16 ones' place in scratch.
+struct HalfPlanes {
+  __half *a_hi, *a_lo, *b_hi, *b_lo;
+  float *a_scale, *b_scale;  // 2^-e, [blocks of K][rows of A / groups of B, padded to whole tiles]
+  int ld;                    // row stride in elements: K rounded up to 8 (TMA wants 16-byte strides)
+  int lda_scale, ldb_scale;
+  Planes tf32;
+  void* extra;
+};
+inline int alloc_half_planes(vtlb_ctx* ctx, int rows_a, int rows_b, int K, size_t extra_bytes, HalfPlanes* p) {
+  p->ld = (int)vtlb_round_up((size_t)K, 8);
+  const size_t blocks = (size_t)(K + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
+  p->lda_scale = (int)vtlb_round_up((size_t)rows_a, 256);
+  p->ldb_scale = (int)vtlb_round_up((size_t)rows_b, 256) / gemm::kHalfGroup;
+  const size_t a = vtlb_round_up((size_t)rows_a * p->ld, 128), b = vtlb_round_up((size_t)rows_b * p->ld, 128);
+  const size_t front = (2 * a + 2 * b) * sizeof(__half);
+  const size_t sa = blocks * p->lda_scale, sb = vtlb_round_up(blocks * p->ldb_scale, 64);
+  if (int rc = alloc_planes(ctx, rows_a, rows_b, K, front + (sa + sb) * sizeof(float) + extra_bytes, &p->tf32)) return rc;
+  p->a_hi = (__half*)p->tf32.a_hi;
+  p->a_lo = p->a_hi + a;
+  p->b_hi = p->a_lo + a;
+  p->b_lo = p->b_hi + b;
+  // the factors lie behind both kinds of planes
+  p->a_scale = (float*)p->tf32.extra;
+  p->b_scale = p->a_scale + sa;
+  p->extra = p->b_scale + sb;
+  return VTLB_OK;
+}
+
 inline int bn_override() {
   static int v = -1;
   if (v < 0) {
@@ -64,43 +102,61 @@ inline int effective_splits(int K, int want) {
   return (total_kb + per - 1) / per;
 }
 
+// Output tensor maps of an epilogue, and which of its extras it can do (`fused`, see launch_tf32x3).
+template <class Epi>
+int prepare_epilogue(vtlb_ctx* ctx, gemm::TmapSet* tm, Epi* epi, int M, int N, int* fused) {
+  if (fused) *fused = 0;
+  if constexpr (Epi::kTmaCapable) {
+    // outputs with a 16-byte-multiple row pitch go out through TMA stores
+    epi->tma = (epi->ldy % 4 == 0) && vtlb_aligned16(epi->Y) && (!epi->pre || vtlb_aligned16(epi->pre)) &&
+              (!epi->bias || N % 4 == 0);
+    if (epi->tma) {
+      int rc0 = gemm::encode_tmap_2d(ctx, &tm->out[0], true, epi->Y, N, M, (uint64_t)epi->ldy * 4, 32, 32);
+      if (rc0) return rc0;
+      tm->out[1] = tm->out[0];
+      if (epi->pre &&
+          (rc0 = gemm::encode_tmap_2d(ctx, &tm->out[1], true, epi->pre, N, M, (uint64_t)epi->ldy * 4, 32, 32)))
+        return rc0;
+    }
+    if constexpr (gemm::EpiHasPlanes<Epi>::value) {
+      // planes of the result leave through TMA stores too; without that path the caller splits
+      // the stored result in a pass of its own
+      if (!epi->tma || N % 4 != 0 || (epi->mask && !vtlb_aligned16(epi->mask))) {
+        epi->planes = 0;
+        epi->mask_fused = 0;
+      } else {
+        epi->mask_fused = epi->mask != nullptr;
+      }
+      if (epi->planes & 1) {
+        int rc0 = gemm::encode_tmap_2d(ctx, &tm->out[2], true, epi->rows_hi, N, M, (uint64_t)epi->ld_rows * 4, 32, 32);
+        if (!rc0) rc0 = gemm::encode_tmap_2d(ctx, &tm->out[3], true, epi->rows_lo, N, M, (uint64_t)epi->ld_rows * 4, 32, 32);
+        if (rc0) return rc0;
+      }
+      if (fused) *fused = (epi->planes ? 1 : 0) | (epi->mask_fused ? 2 : 0);
+    }
+  }
+  return VTLB_OK;
+}
+
+// Operand tensor maps of the CTA-pair kernel on TF32 planes.
+inline int encode_tf32_pair(vtlb_ctx* ctx, gemm::TmapSet* tm, const Planes& p, int M, int N, int K) {
+  const uint64_t stride = (uint64_t)p.ld * 4;
+  int rc = gemm::encode_tmap_2d(ctx, &tm->a[0], true, p.a_hi, K, M, stride, 32, gemm::BM);
+  if (!rc) rc = gemm::encode_tmap_2d(ctx, &tm->a[1], true, p.a_lo, K, M, stride, 32, gemm::BM);
+  if (!rc) rc = gemm::encode_tmap_2d(ctx, &tm->b[0], true, p.b_hi, K, N, stride, 32, 128);
+  if (!rc) rc = gemm::encode_tmap_2d(ctx, &tm->b[1], true, p.b_lo, K, N, stride, 32, 128);
+  return rc;
+}
+
 // D[M,N] = A[M,K] . B[N,K]^T on the planes, epilogue functor `epi`.
 // `fused` (optional) receives bit 0 = the epilogue writes the requested operand planes of the result,
 // bit 1 = it applies the ReLU-backward mask; what it does not do, the caller does in separate passes.
 template <class Epi>
 int launch_tf32x3(vtlb_ctx* ctx, const Planes& p, int M, int N, int K, Epi epi, int splits = 1,
                   int* fused = nullptr) {
-  if (fused) *fused = 0;
   gemm::TmapSet tm;
-  if constexpr (Epi::kTmaCapable) {
-    // outputs with a 16-byte-multiple row pitch go out through TMA stores
-    epi.tma = (epi.ldy % 4 == 0) && vtlb_aligned16(epi.Y) && (!epi.pre || vtlb_aligned16(epi.pre)) &&
-              (!epi.bias || N % 4 == 0);
-    if (epi.tma) {
-      int rc0 = gemm::encode_tmap_2d(ctx, &tm.out[0], true, epi.Y, N, M, (uint64_t)epi.ldy * 4, 32, 32);
-      if (rc0) return rc0;
-      tm.out[1] = tm.out[0];
-      if (epi.pre &&
-          (rc0 = gemm::encode_tmap_2d(ctx, &tm.out[1], true, epi.pre, N, M, (uint64_t)epi.ldy * 4, 32, 32)))
-        return rc0;
-    }
-    if constexpr (gemm::EpiHasPlanes<Epi>::value) {
-      // planes of the result leave through TMA stores too; without that path the caller splits
-      // the stored result in a pass of its own
-      if (!epi.tma || N % 4 != 0 || (epi.mask && !vtlb_aligned16(epi.mask))) {
-        epi.planes = 0;
-        epi.mask_fused = 0;
-      } else {
-        epi.mask_fused = epi.mask != nullptr;
-      }
-      if (epi.planes & 1) {
-        int rc0 = gemm::encode_tmap_2d(ctx, &tm.out[2], true, epi.rows_hi, N, M, (uint64_t)epi.ld_rows * 4, 32, 32);
-        if (!rc0) rc0 = gemm::encode_tmap_2d(ctx, &tm.out[3], true, epi.rows_lo, N, M, (uint64_t)epi.ld_rows * 4, 32, 32);
-        if (rc0) return rc0;
-      }
-      if (fused) *fused = (epi.planes ? 1 : 0) | (epi.mask_fused ? 2 : 0);
-    }
-  }
+  int rc;
+  if ((rc = prepare_epilogue(ctx, &tm, &epi, M, N, fused))) return rc;
   int bn = bn_override();
   if (bn != 64 && bn != 128) {
     const int tiles_m = (M + gemm::BM - 1) / gemm::BM;
@@ -108,7 +164,6 @@ int launch_tf32x3(vtlb_ctx* ctx, const Planes& p, int M, int N, int K, Epi epi, 
     if (N <= 64) bn = 64;
   }
   const uint64_t stride = (uint64_t)p.ld * 4;
-  int rc;
   // large problems: CTA pairs, 256 x 256 tiles (VTLB_F32_PAIR=0 keeps them on single CTAs)
   static int pair_env = -2;
   if (pair_env == -2) {
@@ -116,10 +171,7 @@ int launch_tf32x3(vtlb_ctx* ctx, const Planes& p, int M, int N, int K, Epi epi, 
     pair_env = e ? atoi(e) : -1;
   }
   if (splits == 1 && pair_env != 0 && gemm2::pair_worthwhile(ctx, M, N)) {
-    if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[0], true, p.a_hi, K, M, stride, 32, gemm::BM))) return rc;
-    if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[1], true, p.a_lo, K, M, stride, 32, gemm::BM))) return rc;
-    if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[0], true, p.b_hi, K, N, stride, 32, 128))) return rc;
-    if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[1], true, p.b_lo, K, N, stride, 32, 128))) return rc;
+    if ((rc = encode_tf32_pair(ctx, &tm, p, M, N, K))) return rc;
     return gemm2::launch_pair<gemm::KIND_TF32X3, Epi>(ctx, tm, epi, M, N, K);
   }
   if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[0], true, p.a_hi, K, M, stride, 32, gemm::BM))) return rc;
@@ -128,6 +180,24 @@ int launch_tf32x3(vtlb_ctx* ctx, const Planes& p, int M, int N, int K, Epi epi, 
   if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[1], true, p.b_lo, K, N, stride, 32, bn))) return rc;
   if (bn == 128) return gemm::launch<gemm::KIND_TF32X3, 128, 3, Epi>(ctx, tm, epi, M, N, K, splits);
   return gemm::launch<gemm::KIND_TF32X3, 64, 4, Epi>(ctx, tm, epi, M, N, K, splits);
+}
+
+// The same product on f16 planes, on CTA pairs.  The epilogue hands on no planes.  `epoch` names the split passes.
+template <class Epi>
+int launch_f16x3(vtlb_ctx* ctx, const HalfPlanes& p, int M, int N, int K, Epi epi, uint32_t epoch, int* fused) {
+  gemm::TmapSet tm;
+  int rc;
+  epi.planes = 0;
+  if ((rc = prepare_epilogue(ctx, &tm, &epi, M, N, fused))) return rc;
+  const uint64_t stride = (uint64_t)p.ld * 2, inner = (uint64_t)K * 2;  // bytes
+  if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[0], false, p.a_hi, inner, M, stride, 128, gemm::BM))) return rc;
+  if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[1], false, p.a_lo, inner, M, stride, 128, gemm::BM))) return rc;
+  if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[0], false, p.b_hi, inner, N, stride, 128, 128))) return rc;
+  if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[1], false, p.b_lo, inner, N, stride, 128, 128))) return rc;
+  const gemm::HalfScales sc{p.a_scale, p.b_scale, p.lda_scale, p.ldb_scale, ctx->d_status + vtlb_ctx::kUnfitWord, epoch};
+  if ((rc = gemm2::launch_pair<gemm::KIND_F16X3, Epi>(ctx, tm, epi, M, N, K, 0, false, sc))) return rc;
+  if ((rc = encode_tf32_pair(ctx, &tm, p.tf32, M, N, K))) return rc;
+  return gemm2::launch_pair<gemm::KIND_TF32X3, Epi>(ctx, tm, epi, M, N, K, 0, false, sc);
 }
 
 // Epilogue: y = acc + bias[col] (one f32 add, as the reference's broadcast add on the

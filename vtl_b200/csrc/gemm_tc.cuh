@@ -32,7 +32,7 @@ constexpr int EPI_WARPS = 8;       // two warps per tensor-memory lane quarter, 
 constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
 constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;  // 2 s per wait
 
-enum Kind { KIND_I8 = 0, KIND_TF32X3 = 1 };
+enum Kind { KIND_I8 = 0, KIND_TF32X3 = 1, KIND_F16X3 = 2 };
 
 template <int KIND>
 struct Traits;
@@ -47,6 +47,27 @@ struct Traits<KIND_TF32X3> {
   static constexpr int ELEM = 4;
   static constexpr int NOP = 2;    // hi and lo
   static constexpr uint32_t CFMT = ptx::kCfmtF32, ABFMT = ptx::kFmtTF32;
+};
+
+// f32 operands as two f16 planes of scaled values (f32_common.cuh, struct HalfPlanes)
+template <>
+struct Traits<KIND_F16X3> {
+  static constexpr int ELEM = 2;
+  static constexpr int NOP = 2;    // hi and lo
+  static constexpr uint32_t CFMT = ptx::kCfmtF32, ABFMT = ptx::kFmtF16;
+};
+constexpr int kHalfBlock = 256;    // elements of K that share a scale
+constexpr int kHalfGroup = 32;     // rows of B (columns of D) that share one too: a chunk of the epilogue
+
+// What a product on f16 planes needs beside them: the factors that undo the scaling, a[block of K][row of A] and
+// b[block of K][group of rows of B], and the word by which the split passes say that f16 cannot hold the operands
+// (it then equals `epoch`, and the product is left to the 3xTF32 kernel launched behind it).
+struct HalfScales {
+  const float* a = nullptr;
+  const float* b = nullptr;
+  int lda = 0, ldb = 0;
+  const uint32_t* unfit = nullptr;
+  uint32_t epoch = 0;
 };
 
 struct TmapSet {

@@ -1,5 +1,6 @@
-// GEMM on CTA pairs: tcgen05.mma.cta_group::2, one 256 x 256 tile of D per pair; INT8 (kind::i8)
-// and f32 as 3xTF32 (kind::tf32 on hi/lo planes).
+// GEMM on CTA pairs: tcgen05.mma.cta_group::2, one 256 x 256 tile of D per pair; INT8 (kind::i8),
+// f32 as 3xTF32 (kind::tf32 on hi/lo planes) and f32 as three f16 products (kind::f16 on hi/lo planes
+// of block-scaled values: the same 22 bits per operand at twice the rate and half the bytes).
 //
 // Why a pair: with one CTA per 128 x 256 tile every SM has to land 48 KB of operands in
 // shared memory per 512 tensor-core cycles while the MMA reads 96 B/clk from the same
@@ -33,6 +34,9 @@ constexpr int BN2 = 256;      // columns of D per pair tile
 #define VTLB_PAIR_STAGES 6  // shared-memory ring depth of the INT8 pair kernel (tuning knob)
 #endif
 
+#ifndef VTLB_F16_CHUNK
+#define VTLB_F16_CHUNK 2
+#endif
 template <int KIND>
 struct Cfg {
   static constexpr int NOP = gemm::Traits<KIND>::NOP;                 // operand planes per side
@@ -47,7 +51,11 @@ struct Cfg {
   // see gemm_tc.cuh).  With 256 columns per accumulator and two buffers there is no room in tensor
   // memory for a separate accumulator of the small cross terms: here they share the main one, which
   // costs three truncations per K step instead of one, still two orders inside the error bound.
-  static constexpr int CHUNK_KB = KIND == gemm::KIND_TF32X3 ? 4 : 0;
+  // The f16 planes close it every 2 stages = 128 elements (a stage holds twice the K).  At 4 stages the sums of
+  // 4096 uniform products were off by 1.58e-6 of 64-bit ones where 3xTF32 leaves 1.08e-6; at 2 by 6.8e-7 (normal ones: 4.9e-7 against 9.2e-7).
+  static constexpr int CHUNK_KB = KIND == gemm::KIND_I8 ? 0 : KIND == gemm::KIND_F16X3 ? VTLB_F16_CHUNK : 4;
+  static constexpr int SCALE_KB = gemm::kHalfBlock * 2 / (int)ROW_BYTES;  // stages that share a scale (f16 planes)
+  static_assert(KIND != gemm::KIND_F16X3 || SCALE_KB % CHUNK_KB == 0, "an accumulator has one scale");
 };
 constexpr uint32_t TMEM_COLS = 2 * BN2;
 
@@ -116,6 +124,17 @@ __device__ __forceinline__ void umma_tf32_pair(uint32_t d_tmem, uint64_t adesc, 
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 __device__ __forceinline__ void umma_i8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                              uint32_t accumulate) {
   asm volatile(
@@ -167,13 +186,17 @@ template <int KIND, class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M, int N, int K,
                  int group_m, int a_chunk_k, int split_tiles, uint32_t* ksplit_buf, uint32_t ksplit_epoch,
-                 uint32_t* status) {
+                 uint32_t* status, const gemm::HalfScales sc) {
   using T = gemm::Traits<KIND>;
   using C = Cfg<KIND>;
   constexpr int NOP = C::NOP, STAGES = C::STAGES;
   constexpr int BK = ROW_BYTES / T::ELEM;  // elements of K per stage
+  constexpr int XSTEP = KIND == gemm::KIND_F16X3 ? (int)ROW_BYTES : BK;  // ... in tensor-map coordinates (f16: bytes)
   constexpr int KSTEPS = ROW_BYTES / 32;
   constexpr uint32_t IDESC = ptx::umma_idesc(T::CFMT, T::ABFMT, 2 * BM, BN2);
+
+  // one of the two kernels launched for a product on f16 planes leaves at once; both CTAs of a pair read the same
+  if (KIND != gemm::KIND_I8 && sc.unfit != nullptr && (*sc.unfit == sc.epoch) != (KIND == gemm::KIND_TF32X3)) return;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -293,11 +316,11 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
               tma_load_3d_pair(sa + i * C::A_TILE, &tm.a[i], (kb * BK) % a_chunk_k, m0, (kb * BK) / a_chunk_k,
                                leader_full);
             else
-              tma_load_2d_pair(sa + i * C::A_TILE, &tm.a[i], kb * BK, m0, leader_full);
+              tma_load_2d_pair(sa + i * C::A_TILE, &tm.a[i], kb * XSTEP, m0, leader_full);
           }
 #pragma unroll
           for (int i = 0; i < NOP; ++i)
-            tma_load_2d_pair(sb + i * C::B_HALF, &tm.b[i], kb * BK, n0, leader_full);
+            tma_load_2d_pair(sb + i * C::B_HALF, &tm.b[i], kb * XSTEP, n0, leader_full);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -342,9 +365,15 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
                 const uint64_t a_lo = ptx::umma_desc_k_sw128(sa + C::A_TILE) + 2u * kk;
                 const uint64_t b_hi = ptx::umma_desc_k_sw128(sb) + 2u * kk;
                 const uint64_t b_lo = ptx::umma_desc_k_sw128(sb + C::B_HALF) + 2u * kk;
-                umma_tf32_pair(d_tmem, a_lo, b_hi, IDESC, first);  // small terms first
-                umma_tf32_pair(d_tmem, a_hi, b_lo, IDESC, 1);
-                umma_tf32_pair(d_tmem, a_hi, b_hi, IDESC, 1);
+                if constexpr (KIND == gemm::KIND_F16X3) {
+                  umma_f16_pair(d_tmem, a_lo, b_hi, IDESC, first);  // small terms first
+                  umma_f16_pair(d_tmem, a_hi, b_lo, IDESC, 1);
+                  umma_f16_pair(d_tmem, a_hi, b_hi, IDESC, 1);
+                } else {
+                  umma_tf32_pair(d_tmem, a_lo, b_hi, IDESC, first);
+                  umma_tf32_pair(d_tmem, a_hi, b_lo, IDESC, 1);
+                  umma_tf32_pair(d_tmem, a_hi, b_hi, IDESC, 1);
+                }
               }
             }
             umma_commit_pair(empty_bar(stage));
@@ -446,17 +475,40 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
           }
         }
         for (int kb0 = 0; kb0 < num_kb; kb0 += chunk_kb) {
+          // f16 planes: this row's factors for the warp's four chunks, fetched before the wait (the arrays are
+          // padded to whole tiles: no bounds to check).  Powers of two, and so are their products: the split passes
+          // left operands whose factors could leave the f32 range to the other kernel.
+          float f[BN2 / 64];
+          if constexpr (KIND == gemm::KIND_F16X3) {
+            const int blk = kb0 / C::SCALE_KB;
+            const float fa = __ldg(sc.a + (size_t)blk * sc.lda + row0 + lane);
+#pragma unroll
+            for (int cc = 0; cc < BN2 / 64; ++cc)
+              f[cc] = __fmul_rn(fa, __ldg(sc.b + (size_t)blk * sc.ldb + n0 / gemm::kHalfGroup + 2 * cc + half));
+          }
           ok = ptx::mbar_wait_bounded(tfull_bar(acc), acc_phase, abort_flag, WAIT_LIMIT_NS);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           ptx::tc_fence_after();
 #pragma unroll
-          for (int cc = 0; cc < BN2 / 64; ++cc) {
-            uint32_t v[32];
-            ptx::tmem_ld_32x32(lane_base + acc * BN2 + (2 * cc + half) * 32, v);
+          for (int cc = 0; cc < BN2 / 32; ++cc) {  // 16 columns at a time: the running sums own the registers
+            uint32_t v[16];
+            ptx::tmem_ld_32x16(lane_base + acc * BN2 + (2 * (cc / 2) + half) * 32 + (cc & 1) * 16, v);
             ptx::tmem_wait_ld();
+            if constexpr (KIND == gemm::KIND_F16X3) {
+              // sum += acc * factor, two columns an instruction; the product is exact, only the sum rounds
+              const uint64_t f2 = ptx::f2_pack(f[cc / 2], f[cc / 2]);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) sum[cc * 32 + j] = __fadd_rn(sum[cc * 32 + j], __uint_as_float(v[j]));
+              for (int j = 0; j < 16; j += 2) {
+                float& s0 = sum[cc * 16 + j];
+                float& s1 = sum[cc * 16 + j + 1];
+                const uint64_t a2 = ptx::f2_pack(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+                ptx::f2_unpack(ptx::f2_fma(a2, f2, ptx::f2_pack(s0, s1)), s0, s1);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) sum[cc * 16 + j] = __fadd_rn(sum[cc * 16 + j], __uint_as_float(v[j]));
+            }
           }
           ptx::tc_fence_before();
           __syncwarp();
@@ -506,7 +558,7 @@ inline bool pair_worthwhile(vtlb_ctx* ctx, int M, int N) {
 
 template <int KIND, class Epi>
 int launch_pair(vtlb_ctx* ctx, const gemm::TmapSet& tm, const Epi& epi, int M, int N, int K,
-                int a_chunk_k = 0, bool k_split = false) {
+                int a_chunk_k = 0, bool k_split = false, const gemm::HalfScales& sc = gemm::HalfScales()) {
   using C = Cfg<KIND>;
   static_assert(C::SMEM_TOTAL <= 232448, "shared memory budget");
   auto kern = gemm_pair_kernel<KIND, Epi>;
@@ -518,7 +570,9 @@ int launch_pair(vtlb_ctx* ctx, const gemm::TmapSet& tm, const Epi& epi, int M, i
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN2 - 1) / BN2);
   int pairs = ctx->sm_count / 2;
   if (tiles < pairs) pairs = tiles;
-  const bool timed = ctx->prof_on && ctx->prof_ev && ctx->prof_n < vtlb_ctx::kProfSlots;
+  // (a 3xTF32 launch behind a product on f16 planes is that product once more, if at all)
+  const bool timed = ctx->prof_on && ctx->prof_ev && ctx->prof_n < vtlb_ctx::kProfSlots &&
+                     !(KIND == gemm::KIND_TF32X3 && sc.unfit);
   if (timed) cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n], ctx->stream);
   const int group_m = gemm::pick_group_m((M + 2 * BM - 1) / (2 * BM),
                                          (size_t)2 * BM * K * gemm::Traits<KIND>::ELEM * C::NOP);
@@ -533,7 +587,7 @@ int launch_pair(vtlb_ctx* ctx, const gemm::TmapSet& tm, const Epi& epi, int M, i
   if (split_tiles && ++ctx->ksplit_epoch == 0) ctx->ksplit_epoch = 1;  // flags hold the epoch of their launch
   kern<<<2 * pairs, NUM_THREADS, C::SMEM_TOTAL, ctx->stream>>>(tm, epi, M, N, K, group_m, a_chunk_k, split_tiles,
                                                                (uint32_t*)ctx->ksplit_buf, ctx->ksplit_epoch,
-                                                               ctx->d_status);
+                                                               ctx->d_status, sc);
   if (timed) {
     cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n + 1], ctx->stream);
     ctx->prof_n++;
