@@ -48,3 +48,16 @@ def _check(dev, B, C, H, W, O, k, pad, stride, relu=True, bias=True):
 ])
 def test_strided_windows(dev, B, C, H, W, O, k, pad, stride):
     _check(dev, B, C, H, W, O, k, pad, stride)
+
+
+@pytest.mark.parametrize("B,C,H,W,O,k,pad", [
+    (1, 1, 5, 5, 1, 5, 0), (65, 1, 28, 28, 8, 3, 1),              # one pixel; more images than a wave
+    (3, 3, 9, 7, 5, 3, 0), (2, 2, 13, 11, 9, 5, 2), (2, 4, 6, 6, 13, 1, 0),   # nothing divides
+    (2, 3, 8, 126, 12, 3, 2), (1, 2, 3, 127, 6, 3, 2), (1, 3, 4, 300, 4, 3, 1),  # rows of 128, 129 and 300 outputs
+    (4, 2, 7, 9, 6, 3, 3), (2, 3, 6, 5, 4, 1, 2), (2, 1, 4, 4, 3, 5, 6),      # more padding than the window covers
+    (16, 8, 28, 28, 16, 5, 0), (2, 64, 14, 14, 3, 5, 2), (2, 70, 5, 5, 2, 5, 0),  # slices and stages of channels
+    (50, 20, 12, 12, 50, 5, 0), (16, 3, 32, 32, 33, 3, 1),        # CTAs that share the channels
+])
+@pytest.mark.parametrize("relu,bias", [(True, True), (False, False)])
+def test_small_products_on_cuda_cores(dev, B, C, H, W, O, k, pad, relu, bias):
+    _check(dev, B, C, H, W, O, k, pad, 1, relu, bias)

@@ -11,6 +11,7 @@
 //   d_weight: dW[oc, k]        = gT[oc, m] . colT[k, m]^T      (split-K over m = (b,oh,ow))
 //   d_input : dcolT[k, m]      = Wt[k, oc] . gM[m, oc]^T, then a col2im gather
 //   d_bias  : per-channel sums of g (f64 partials)
+#include "conv_direct.cuh"
 #include "conv_igemm.cuh"
 #include "conv_slab.cuh"
 #include "conv_wgrad.cuh"
@@ -518,15 +519,23 @@ int conv2d_fwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_x, const void* 
   const int M = (int)d.M(), K = d.K();
   f32::Planes p;
   if (dh == 1 && dw == 1 && use_igemm(K) && igemm_taps_ok(kh, kw)) {  // dilated windows take the lowered route
+    const igemm::Geometry g{B, C, H, W, d.OH, d.OW, sh, sw, kh, kw, -ph, -pw, 1, K};
+    cslab::Tiling tl;
+    const bool slab = cslab::usable(g, &tl) && vtlb_aligned16(d_y) && (!d_pre_or_null || vtlb_aligned16(d_pre_or_null));
+    if (cdirect::worthwhile(ctx, g, slab ? &tl : nullptr, O)) {
+      cdirect::Params q = {};
+      q.src = (const float*)d_x, q.w = (const float*)d_w, q.bias = (const float*)d_bias_or_null;
+      q.dst = (float*)d_y, q.pre = (float*)d_pre_or_null;
+      q.B = B, q.Cs = C, q.Hs = H, q.Ws = W, q.Cd = O, q.Hd = d.OH, q.Wd = d.OW;
+      q.oy = -ph, q.ox = -pw, q.relu = relu;
+      return cdirect::launch_direct(ctx, q, kh);
+    }
     if ((rc = f32::alloc_planes(ctx, 0, O, K, 0, &p))) return rc;
     VTLB_CUDA(ctx, vtlb_launch_early(regroup_weights_split_kernel, dim3(f32::grid_for(ctx, (size_t)O * K, 256)), dim3(256),
                                      0, ctx->stream, (const float*)d_w, O, C, kh * kw, 0, p.ld, p.b_hi, p.b_lo));
     VTLB_LAUNCHED(ctx);
-    const igemm::Geometry g{B, C, H, W, d.OH, d.OW, sh, sw, kh, kw, -ph, -pw, 1, K};
     EpiConvOut epi{(float*)d_y, (const float*)d_bias_or_null, (float*)d_pre_or_null, O, d.P(), relu};
-    cslab::Tiling tl;
-    if (cslab::usable(g, &tl) && vtlb_aligned16(d_y) && (!d_pre_or_null || vtlb_aligned16(d_pre_or_null)))
-      return cslab::launch(ctx, (const float*)d_x, g, tl, p.b_hi, p.b_lo, p.ld, epi, O);
+    if (slab) return cslab::launch(ctx, (const float*)d_x, g, tl, p.b_hi, p.b_lo, p.ld, epi, O);
     return igemm::launch(ctx, (const float*)d_x, g, p.b_hi, p.b_lo, p.ld, epi, M, O);
   }
   if ((rc = f32::alloc_planes(ctx, M, O, K, 0, &p))) return rc;
@@ -554,7 +563,13 @@ int conv2d_bwd_impl(vtlb_ctx* ctx, const void* d_g, const void* d_x, const void*
   if (!d_g) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_conv2d_bwd_f32: null gradient");
   const int M = (int)d.M(), K = d.K(), P = d.P();
   const float* g = (const float*)d_g;
-  if (d_dw_or_null && cwgrad::usable(sh, sw, kh, kw, d.OW, dilated ? 2 : 1)) {
+  const bool pixel_kernel = cwgrad::usable(sh, sw, kh, kw, d.OW, dilated ? 2 : 1);
+  if (d_dw_or_null && !dilated && cdirect::wgrad_worthwhile(ctx, B, C, O, d.OH, d.OW, kh, kw, pixel_kernel)) {
+    if (!d_x) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_conv2d_bwd_f32: d_weight needs x");
+    if ((rc = cdirect::launch_wgrad(ctx, g, (const float*)d_x, (float*)d_dw_or_null, B, C, H, W, O, d.OH, d.OW, kh, ph,
+                                    pw, sh, sw)))
+      return rc;
+  } else if (d_dw_or_null && pixel_kernel) {
     // unit stride, window at most 3 x 3, output rows of at most 32 pixels: the implicit GEMM over pixels
     if (!d_x) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_conv2d_bwd_f32: d_weight needs x");
     const int parts = cwgrad::parts_for(ctx, B, C, O, d.OH);
@@ -603,18 +618,26 @@ int conv2d_bwd_impl(vtlb_ctx* ctx, const void* d_g, const void* d_x, const void*
     // dx[(b, ih, iw), ic] = sum over (oc, a, b) of g[b][oc][ih + ph - a][iw + pw - b] * W[oc][ic][a][b]
     if (!d_w) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_conv2d_bwd_f32: d_input needs the weights");
     const int Kd = O * kh * kw;
-    f32::Planes p;
-    if ((rc = f32::alloc_planes(ctx, 0, C, Kd, 0, &p))) return rc;
-    VTLB_CUDA(ctx, vtlb_launch_early(regroup_weights_split_kernel, dim3(f32::grid_for(ctx, (size_t)O * C * kh * kw, 256)),
-                                     dim3(256), 0, ctx->stream, (const float*)d_w, O, C, kh * kw, 1, p.ld, p.b_hi, p.b_lo));
-    VTLB_LAUNCHED(ctx);
     const igemm::Geometry gg{B, O, d.OH, d.OW, H, W, 1, 1, kh, kw, ph, pw, -1, Kd};
-    EpiConvOut epi{(float*)d_dx_or_null, nullptr, nullptr, C, H * W, 0};
     cslab::Tiling tl;
-    if (cslab::usable(gg, &tl) && vtlb_aligned16(d_dx_or_null))
-      rc = cslab::launch(ctx, g, gg, tl, p.b_hi, p.b_lo, p.ld, epi, C);
-    else
-      rc = igemm::launch(ctx, g, gg, p.b_hi, p.b_lo, p.ld, epi, B * H * W, C);
+    const bool slab = cslab::usable(gg, &tl) && vtlb_aligned16(d_dx_or_null);
+    if (cdirect::worthwhile(ctx, gg, slab ? &tl : nullptr, C)) {
+      cdirect::Params q = {};
+      q.src = g, q.w = (const float*)d_w, q.dst = (float*)d_dx_or_null;
+      q.B = B, q.Cs = O, q.Hs = d.OH, q.Ws = d.OW, q.Cd = C, q.Hd = H, q.Wd = W;
+      q.oy = ph - (kh - 1), q.ox = pw - (kw - 1), q.mirror = 1;
+      rc = cdirect::launch_direct(ctx, q, kh);
+    } else {
+      f32::Planes p;
+      if ((rc = f32::alloc_planes(ctx, 0, C, Kd, 0, &p))) return rc;
+      VTLB_CUDA(ctx, vtlb_launch_early(regroup_weights_split_kernel,
+                                       dim3(f32::grid_for(ctx, (size_t)O * C * kh * kw, 256)), dim3(256), 0, ctx->stream,
+                                       (const float*)d_w, O, C, kh * kw, 1, p.ld, p.b_hi, p.b_lo));
+      VTLB_LAUNCHED(ctx);
+      EpiConvOut epi{(float*)d_dx_or_null, nullptr, nullptr, C, H * W, 0};
+      rc = slab ? cslab::launch(ctx, g, gg, tl, p.b_hi, p.b_lo, p.ld, epi, C)
+                : igemm::launch(ctx, g, gg, p.b_hi, p.b_lo, p.ld, epi, B * H * W, C);
+    }
     if (rc) return rc;
   } else if (d_dx_or_null) {  // dcolT[k, m] = sum_oc W[oc, k] * g[m, oc]; dx = col2im(dcolT)
     if (!d_w) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_conv2d_bwd_f32: d_input needs the weights");
