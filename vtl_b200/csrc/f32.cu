@@ -586,6 +586,11 @@ int linear_fwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_X, const void* 
                        (const float*)d_b_or_null, relu, (float*)d_pre_or_null, ex);
 }
 
+bool overlap(const void* a, size_t na, const void* b, size_t nb) {  // arrays of f32
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + nb * sizeof(float) && y < x + na * sizeof(float);
+}
+
 int linear_bwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_G, const void* d_X, const void* d_W,
                     void* d_dX_or_null, void* d_dW_or_null, void* d_db_or_null, int M, int N, int K,
                     const vtlb_planes* g_rows, const vtlb_planes* g_cols, const vtlb_planes* x_cols,
@@ -616,6 +621,21 @@ int linear_bwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_G, const void* 
     d_dW_or_null = nullptr;
     d_db_or_null = nullptr;
   }
+  bool db_done = false;
+  // a small layer: both products in one launch, where neither writes what the other reads
+  if (narrow && d_dX_or_null && d_dW_or_null && d_W && d_X && vtlb_aligned16(d_dX_or_null) && vtlb_aligned16(d_dW_or_null) &&
+      !overlap(d_dX_or_null, (size_t)M * K, d_X, (size_t)M * K) && !overlap(d_dX_or_null, (size_t)M * K, d_G, (size_t)M * N) &&
+      !overlap(d_dW_or_null, (size_t)N * K, d_W, (size_t)N * K) && !overlap(d_dW_or_null, (size_t)N * K, d_G, (size_t)M * N) &&
+      !(d_relu_mask_src_or_null && overlap(d_dW_or_null, (size_t)N * K, d_relu_mask_src_or_null, (size_t)M * K)) &&
+      !(d_db_or_null && (overlap(d_db_or_null, (size_t)N, d_W, (size_t)N * K) ||
+                         overlap(d_db_or_null, (size_t)N, d_G, (size_t)M * N)))) {
+    bool done = false;
+    if ((rc = f32::sgemm_small_linear_bwd(ctx, (const float*)d_G, (const float*)d_X, (const float*)d_W,
+                                          (float*)d_dX_or_null, (float*)d_dW_or_null, (float*)d_db_or_null, M, N, K,
+                                          (const float*)d_relu_mask_src_or_null, &done, &db_done)))
+      return rc;
+    if (done) d_dX_or_null = d_dW_or_null = nullptr;
+  }
   if (d_dX_or_null) {  // dX[M,K] = G[M,N] . W[N,K]   (then, optionally, ReLU backward of the layer below)
     if (!d_W) return vtlb_fail(ctx, VTLB_EINVAL, "%s: dX needs W", fn);
     GemmExtras ex;
@@ -627,7 +647,6 @@ int linear_bwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_G, const void* 
                             0, nullptr, ex)))
       return rc;
   }
-  bool db_done = false;
   if (d_dW_or_null) {  // dW[N,K] = G^T[N,M] . X[M,K]
     if (!d_X) return vtlb_fail(ctx, VTLB_EINVAL, "%s: dW needs X", fn);
     if (d_db_or_null && 2.0 * M * N * K <= ctx->small_gemm_flops && vtlb_aligned16(d_dW_or_null)) {

@@ -347,6 +347,12 @@ int sgemm_small(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, cons
                 const float* B, float* C, const float* bias, int relu, float* pre,
                 float* a_rowsum = nullptr, bool* rowsum_done = nullptr, const float* mask = nullptr);
 
+// Both products of a small Linear backward in one launch: dX[M,K] = G.W (zeroed where mask < 0, mask may be null) and
+// dW[N,K] = G^T.X, with db = column sums of G where that costs nothing (*db_done).  *done = false: nothing was
+// launched, the products are too long in K for it.
+int sgemm_small_linear_bwd(vtlb_ctx* ctx, const float* G, const float* X, const float* W, float* dX, float* dW, float* db,
+                           int M, int N, int K, const float* mask, bool* done, bool* db_done);
+
 // Linear layers with at most 16 output features and at least 2048 inputs (linear_narrow.cu): Y = X.W^T + b,
 // dX = G.W, dW = G^T.X with db = column sums of G (either of dW / db may be null), each streaming its
 // long operand once.  narrow_linear_ok checks shape and the alignment of the three long operands.

@@ -42,11 +42,6 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)
 __device__ __forceinline__ void cp_async_f32(uint32_t dst, const float* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
@@ -57,38 +52,43 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, f
                : "memory");
 }
 
-// grid = (tiles_n, tiles_m, splits).  With splits == 1 the epilogue is applied here and C is
-// written.  With `cluster` set the launch has cluster dimensions (1, 1, splits) and the partial
-// sums are exchanged through shared memory; otherwise they go to partial[z][M][N].
+// One product: C[M,N] = op(A).op(B) with its epilogue, cut into `splits` ranges of kps along K.  With `cluster` the
+// ranges of a tile are the CTAs of a thread-block cluster, which exchange the partial sums through shared memory;
+// else, with more than one range, they go to partial[z][M][N].
+struct SmallProduct {
+  const float *A, *B;
+  float* C;
+  const float* bias;
+  float* pre;
+  int M, N, K, kps, splits, relu, cluster;
+  float* partial;
+  float* a_rowsum;
+  const float* mask;
+};
+struct SmallShared {
+  // landing zone of the cluster exchange: [source CTA][owned row][TN]; written by the peers
+  // while this CTA may still be in its K loop, so it shares nothing with the stages
+  float land[kLandRows][TN];
+};
+
+// The tile (bx, by) of p, range z.  TA, TB: A is stored [K, M], B is stored [N, K].
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) sgemm_small_kernel(const float* __restrict__ A,
-                                                          const float* __restrict__ B,
-                                                          float* __restrict__ C,
-                                                          const float* __restrict__ bias,
-                                                          float* __restrict__ pre, int M, int N, int K,
-                                                          int k_per_split, int relu,
-                                                          float* __restrict__ partial, int cluster,
-                                                          float* __restrict__ a_rowsum,
-                                                          const float* __restrict__ mask) {
+__device__ __forceinline__ void small_product_tile(const SmallProduct& p, int bx, int by, int z, float* stage_mem,
+                                                   SmallShared& sh) {
+  const float* __restrict__ A = p.A;
+  const float* __restrict__ B = p.B;
+  float* __restrict__ C = p.C;
+  const float* __restrict__ bias = p.bias;
+  float* __restrict__ pre = p.pre;
+  const float* __restrict__ mask = p.mask;
+  const int M = p.M, N = p.N, K = p.K, relu = p.relu, k_per_split = p.kps;
   // NST stages of (A tile [TK][TM+1], B tile [TK][TN+4]) in dynamic shared memory, filled by
   // cp.async: the loads of up to NST K steps (a whole K range) are in flight at once, so
   // a CTA pays one global-memory latency, not one per step
-  extern __shared__ __align__(16) float stage_mem[];
-  // landing zone of the cluster exchange: [source CTA][owned row][TN]; written by the peers
-  // while this CTA may still be in its K loop, so it shares nothing with the stages
-  __shared__ __align__(16) float Land[kLandRows][TN];
-  // "this CTA runs": entered here, waited for before the first store into a peer's memory
-  if (cluster) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-  // Launched with programmatic stream serialisation: the CTAs may be resident before the kernel
-  // in front of this one in the stream has finished (its launch latency hidden behind that
-  // kernel's tail); nothing of that kernel's output is touched before this wait, which returns
-  // once it has completed and its writes are visible.  Then let the next kernel do the same.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x;
   const int ty = tid >> 4, tx = tid & 15;  // 16 x 16 threads, 2 x 4 outputs each
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-  const int kbeg = blockIdx.z * k_per_split;
+  const int m0 = by * TM, n0 = bx * TN;
+  const int kbeg = z * k_per_split;
   const int kend = kbeg + k_per_split < K ? kbeg + k_per_split : K;
   const int nsteps = kend > kbeg ? (kend - kbeg + TK - 1) / TK : 0;
   auto load_stage = [&](int st, int k0) {
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(256) sgemm_small_kernel(const float* __restric
   // f64 and rounded once.  For dW = G^T . X these are the column sums of G, the bias gradient,
   // which would otherwise cost a launch of its own; the first column of tiles computes them from
   // the A tiles it loads anyway.
-  const bool want_sum = a_rowsum != nullptr && blockIdx.x == 0;
+  const bool want_sum = p.a_rowsum != nullptr && bx == 0;
   double rsum0 = 0.0, rsum1 = 0.0;
   for (int s = 0; s < nsteps; ++s) {
     asm volatile("cp.async.wait_group %0;" ::"n"(NST - 1) : "memory");
@@ -154,18 +154,17 @@ __global__ void __launch_bounds__(256) sgemm_small_kernel(const float* __restric
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   if (want_sum && tx == 0) {
-    if (m0 + ty * 2 < M) a_rowsum[m0 + ty * 2] = (float)rsum0;
-    if (m0 + ty * 2 + 1 < M) a_rowsum[m0 + ty * 2 + 1] = (float)rsum1;
+    if (m0 + ty * 2 < M) p.a_rowsum[m0 + ty * 2] = (float)rsum0;
+    if (m0 + ty * 2 + 1 < M) p.a_rowsum[m0 + ty * 2 + 1] = (float)rsum1;
   }
-  if (cluster) {
-    const int S = gridDim.z;
-    const int z = (int)cluster_rank();  // = blockIdx.z: the cluster spans the whole z extent of the grid
+  if (p.cluster) {
+    const int S = p.splits;  // z is this CTA's rank
     const int rows_per = (TM + S - 1) / S;
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every peer has started
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       const int m = ty * 2 + r;  // row of the tile: owner m % S keeps it as its row m / S
-      const uint32_t dst = map_to_rank(smem_addr(&Land[(int)blockIdx.z * rows_per + m / S][tx * 4]), (uint32_t)(m % S));
+      const uint32_t dst = map_to_rank(smem_addr(&sh.land[z * rows_per + m / S][tx * 4]), (uint32_t)(m % S));
       st_cluster_v4(dst, acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -175,8 +174,8 @@ __global__ void __launch_bounds__(256) sgemm_small_kernel(const float* __restric
       const int ml = slot * S + z;
       const int m = m0 + ml, n = n0 + nl;
       if (ml >= TM || m >= M || n >= N) continue;
-      float s0 = Land[slot][nl];
-      for (int r = 1; r < S; ++r) s0 = __fadd_rn(s0, Land[r * rows_per + slot][nl]);
+      float s0 = sh.land[slot][nl];
+      for (int r = 1; r < S; ++r) s0 = __fadd_rn(s0, sh.land[r * rows_per + slot][nl]);
       small_epilogue(s0, m, n, N, bias, pre, relu, C, mask);
     }
     return;
@@ -189,12 +188,56 @@ __global__ void __launch_bounds__(256) sgemm_small_kernel(const float* __restric
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
       if (n >= N) continue;
-      if (partial)
-        partial[((size_t)blockIdx.z * M + m) * N + n] = acc[r][j];
+      if (p.partial)
+        p.partial[((size_t)z * M + m) * N + n] = acc[r][j];
       else
         small_epilogue(acc[r][j], m, n, N, bias, pre, relu, C, mask);
     }
   }
+}
+
+// Launched with programmatic stream serialisation: the CTAs may be resident before the kernel
+// in front of this one in the stream has finished (its launch latency hidden behind that
+// kernel's tail); nothing of that kernel's output is touched before the wait, which returns
+// once it has completed and its writes are visible.  Then let the next kernel do the same.
+// A cluster's first barrier ("this CTA runs") is entered before it, and waited for before the first store into a
+// peer's memory.
+__device__ __forceinline__ void small_prologue(bool cluster) {
+  if (cluster) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// grid = (tiles_n, tiles_m, splits), cluster dimensions (1, 1, splits) with p.cluster.
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(256) sgemm_small_kernel(const __grid_constant__ SmallProduct p) {
+  extern __shared__ __align__(16) float stage_mem[];
+  __shared__ __align__(16) SmallShared sh;
+  small_prologue(p.cluster != 0);
+  small_product_tile<TA, TB>(p, blockIdx.x, blockIdx.y, blockIdx.z, stage_mem, sh);
+}
+
+// The two products of a Linear layer's backward in one launch: dX = G . W and dW = G^T . X, which do not depend on
+// one another.  At 64 x 256 x 784 each is a few microseconds of latency on a part of the SMs, and the second used to
+// wait for the first.  1-D grid in clusters of S CTAs, the first `x_clusters` for dX.  A product cut into S ranges
+// gives a cluster a tile; one that is not cut gives each CTA a tile of its own.
+__global__ void __launch_bounds__(256) sgemm_small_pair_kernel(const __grid_constant__ SmallProduct x,
+                                                               const __grid_constant__ SmallProduct w, int S,
+                                                               int x_clusters) {
+  extern __shared__ __align__(16) float stage_mem[];
+  __shared__ __align__(16) SmallShared sh;
+  const int r = blockIdx.x % S;
+  int c = blockIdx.x / S;
+  const bool first = c < x_clusters;
+  const SmallProduct& p = first ? x : w;
+  if (!first) c -= x_clusters;
+  small_prologue(p.cluster != 0);
+  const int tile = p.cluster ? c : c * S + r, z = p.cluster ? r : 0;
+  const int tiles_n = (p.N + TN - 1) / TN, tiles_m = (p.M + TM - 1) / TM;
+  if (tile >= tiles_n * tiles_m) return;  // of an uncut product only
+  const int by = tile / tiles_n, bx = tile - by * tiles_n;
+  if (first) small_product_tile<false, false>(x, bx, by, z, stage_mem, sh);
+  else small_product_tile<true, false>(w, bx, by, z, stage_mem, sh);
 }
 
 __global__ void __launch_bounds__(256) small_reduce_kernel(const float* __restrict__ partial, int splits,
@@ -212,13 +255,12 @@ __global__ void __launch_bounds__(256) small_reduce_kernel(const float* __restri
 
 }  // namespace
 
-int f32::sgemm_small(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, const float* A,
-                     const float* B, float* C, const float* bias, int relu, float* pre, float* a_rowsum,
-                     bool* rowsum_done, const float* mask) {
-  const int tiles = ((N + TN - 1) / TN) * ((M + TM - 1) / TM);
-  // K ranges of `kps_want` (VTLB_SMALL_KPS overrides): the product is spread over as many SMs as
-  // the cluster limit of 8 ranges allows, since a CTA that walks a long K alone is bound by its own
-  // shared-memory reads (measured on config 1: no split 100 us per step, ranges of 256 80 us, of 128 74 us, of 64 67.5 us)
+namespace {
+
+// K ranges of `kps_want` (VTLB_SMALL_KPS overrides): the product is spread over as many SMs as
+// the cluster limit of 8 ranges allows, since a CTA that walks a long K alone is bound by its own
+// shared-memory reads (measured on config 1: no split 100 us per step, ranges of 256 80 us, of 128 74 us, of 64 67.5 us)
+int pick_splits(vtlb_ctx* ctx, int tiles, int K, int* kps_out) {
   static int kps_want = -1;
   if (kps_want < 0) {
     const char* e = getenv("VTLB_SMALL_KPS");
@@ -229,7 +271,58 @@ int f32::sgemm_small(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K,
   while (splits > 1 && tiles * splits > 4 * ctx->sm_count) --splits;
   int kps = (K + splits - 1) / splits;
   kps = (kps + TK - 1) / TK * TK;
-  splits = (K + kps - 1) / kps;
+  *kps_out = kps;
+  return (K + kps - 1) / kps;
+}
+int tiles_of(int M, int N) { return ((N + TN - 1) / TN) * ((M + TM - 1) / TM); }
+
+int configure_small(vtlb_ctx* ctx) {
+  static std::atomic<uint64_t> configured{0};  // one bit per device
+  if (configured.load(std::memory_order_relaxed) >> (ctx->device & 63) & 1) return VTLB_OK;
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_kernel<false, false>, attr, kStageBytes));
+  VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_kernel<false, true>, attr, kStageBytes));
+  VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_kernel<true, false>, attr, kStageBytes));
+  VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_kernel<true, true>, attr, kStageBytes));
+  VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_pair_kernel, attr, kStageBytes));
+  configured.fetch_or(1ull << (ctx->device & 63), std::memory_order_relaxed);
+  return VTLB_OK;
+}
+
+// Launch in clusters of `cluster` CTAs along x or z, early behind the kernel in front.
+template <typename... KArgs, typename... Args>
+int launch_small(vtlb_ctx* ctx, void (*kern)(KArgs...), dim3 grid, int cluster, bool along_x, Args... args) {
+  static int pdl = -1;  // VTLB_SMALL_PDL=0 switches the early launch off (measurements)
+  if (pdl < 0) {
+    const char* e = getenv("VTLB_SMALL_PDL");
+    pdl = e ? atoi(e) != 0 : 1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = kStageBytes;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)(along_x ? cluster : 1);
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = (unsigned)(along_x ? 1 : cluster);
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 2 : 1;
+  VTLB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, args...));
+  VTLB_LAUNCHED(ctx);
+  return VTLB_OK;
+}
+
+}  // namespace
+
+int f32::sgemm_small(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, const float* A,
+                     const float* B, float* C, const float* bias, int relu, float* pre, float* a_rowsum,
+                     bool* rowsum_done, const float* mask) {
+  SmallProduct p{A, B, C, bias, pre, M, N, K, 0, 1, relu, 0, nullptr, a_rowsum, mask};
+  p.splits = pick_splits(ctx, tiles_of(M, N), K, &p.kps);
   // A few ranges more than a cluster holds (config 1's first layer: K = 784 = 13 ranges of 64) go
   // through the partial buffer and a second launch.  VTLB_SMALL_CLUSTER_CAP=1 makes the ranges long
   // enough to fit one cluster instead, which saves that launch and measured slower (config 1: 46.6
@@ -239,62 +332,60 @@ int f32::sgemm_small(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K,
     const char* e = getenv("VTLB_SMALL_CLUSTER_CAP");
     cap = e ? atoi(e) != 0 : 0;
   }
-  if (cap && splits > kMaxClusterSplits && splits <= 2 * kMaxClusterSplits) {
-    kps = ((K + kMaxClusterSplits - 1) / kMaxClusterSplits + TK - 1) / TK * TK;
-    splits = (K + kps - 1) / kps;
+  if (cap && p.splits > kMaxClusterSplits && p.splits <= 2 * kMaxClusterSplits) {
+    p.kps = ((K + kMaxClusterSplits - 1) / kMaxClusterSplits + TK - 1) / TK * TK;
+    p.splits = (K + p.kps - 1) / p.kps;
   }
-  const bool cluster = splits > 1 && splits <= kMaxClusterSplits;
-  if (splits > 1) a_rowsum = nullptr;  // the by-product needs the whole K in one CTA
-  if (rowsum_done) *rowsum_done = a_rowsum != nullptr;
-  float* partial = nullptr;
-  if (splits > 1 && !cluster) {
+  p.cluster = p.splits > 1 && p.splits <= kMaxClusterSplits;
+  if (p.splits > 1) p.a_rowsum = nullptr;  // the by-product needs the whole K in one CTA
+  if (rowsum_done) *rowsum_done = p.a_rowsum != nullptr;
+  int rc;
+  if (p.splits > 1 && !p.cluster) {
     void* scr = nullptr;
-    int rc = vtlb_scratch(ctx, (size_t)splits * M * N * sizeof(float), &scr);
-    if (rc) return rc;
-    partial = (float*)scr;
+    if ((rc = vtlb_scratch(ctx, (size_t)p.splits * M * N * sizeof(float), &scr))) return rc;
+    p.partial = (float*)scr;
   }
-  dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, splits);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = kStageBytes;
-  cfg.stream = ctx->stream;
-  static std::atomic<uint64_t> configured{0};  // one bit per device
-  if (!(configured.load(std::memory_order_relaxed) >> (ctx->device & 63) & 1)) {
-    VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes));
-    VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes));
-    VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes));
-    VTLB_CUDA(ctx, cudaFuncSetAttribute(sgemm_small_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes));
-    configured.fetch_or(1ull << (ctx->device & 63), std::memory_order_relaxed);
-  }
-  static int pdl = -1;  // VTLB_SMALL_PDL=0 switches the early launch off (measurements)
-  if (pdl < 0) {
-    const char* e = getenv("VTLB_SMALL_PDL");
-    pdl = e ? atoi(e) != 0 : 1;
-  }
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 1;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = (unsigned)(cluster ? splits : 1);
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = pdl ? 2 : 1;
-#define VTLB_SMALL(TA, TB)                                                                               \
-  VTLB_CUDA(ctx, cudaLaunchKernelEx(&cfg, sgemm_small_kernel<TA, TB>, A, B, C, bias, pre, M, N, K, kps, relu, \
-                                    partial, (int)cluster, a_rowsum, mask))
-  if (transA && transB) VTLB_SMALL(true, true);
-  else if (transA) VTLB_SMALL(true, false);
-  else if (transB) VTLB_SMALL(false, true);
-  else VTLB_SMALL(false, false);
-#undef VTLB_SMALL
-  VTLB_LAUNCHED(ctx);
-  if (splits > 1 && !cluster) {
+  if ((rc = configure_small(ctx))) return rc;
+  const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, p.splits);
+  auto kern = transA ? (transB ? sgemm_small_kernel<true, true> : sgemm_small_kernel<true, false>)
+                     : (transB ? sgemm_small_kernel<false, true> : sgemm_small_kernel<false, false>);
+  if ((rc = launch_small(ctx, kern, grid, p.cluster ? p.splits : 1, false, p))) return rc;
+  if (p.partial) {
     VTLB_CUDA(ctx, vtlb_launch_early(small_reduce_kernel, dim3((M * N + 255) / 256), dim3(256), 0, ctx->stream,
-                                     (const float*)partial, splits, M, N, bias, pre, relu, C, mask));
+                                     (const float*)p.partial, p.splits, M, N, bias, pre, relu, C, mask));
     VTLB_LAUNCHED(ctx);
   }
+  return VTLB_OK;
+}
+
+int f32::sgemm_small_linear_bwd(vtlb_ctx* ctx, const float* G, const float* X, const float* W, float* dX, float* dW,
+                                float* db, int M, int N, int K, const float* mask, bool* done, bool* db_done) {
+  *done = false;
+  *db_done = false;
+  SmallProduct x{G, W, dX, nullptr, nullptr, M, K, N, 0, 1, 0, 0, nullptr, nullptr, mask};
+  SmallProduct w{G, X, dW, nullptr, nullptr, N, K, M, 0, 1, 0, 0, nullptr, db, nullptr};
+  const int x_tiles = tiles_of(M, K), w_tiles = tiles_of(N, K);
+  x.splits = pick_splits(ctx, x_tiles, N, &x.kps);
+  w.splits = pick_splits(ctx, w_tiles, M, &w.kps);
+  const int S = x.splits > w.splits ? x.splits : w.splits;
+  if (S > kMaxClusterSplits) return VTLB_OK;  // the partial sums would go through memory
+  for (SmallProduct* p : {&x, &w}) {
+    if (p->splits > 1 && p->splits < S) {  // the cluster's size for both: shorter ranges, the last ones may be empty
+      p->splits = S;
+      p->kps = ((p->K + S - 1) / S + TK - 1) / TK * TK;
+    }
+    p->cluster = p->splits > 1;
+  }
+  if (w.splits > 1) w.a_rowsum = nullptr;
+  const int x_clusters = x.cluster ? x_tiles : (x_tiles + S - 1) / S;
+  const int w_clusters = w.cluster ? w_tiles : (w_tiles + S - 1) / S;
+  int rc;
+  if ((rc = configure_small(ctx))) return rc;
+  if ((rc = launch_small(ctx, sgemm_small_pair_kernel, dim3((unsigned)((x_clusters + w_clusters) * S)), S, true, x, w, S,
+                         x_clusters)))
+    return rc;
+  *done = true;
+  *db_done = w.a_rowsum != nullptr;
   return VTLB_OK;
 }
 
