@@ -130,7 +130,8 @@ int vtlb_gemm_f32(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
 
 /* f32 products of at most `max_flops` (2*M*N*K) run as one FFMA kernel on CUDA cores straight
  * from the caller's operands instead of the tensor-core path: at the size of a 784->256->10
- * MLP on a batch of 64 the call is bound by launch latency, not arithmetic.  Default 1.4e8;
+ * MLP on a batch of 64 the call is bound by launch latency, not arithmetic.  Default 1.4e8, and
+ * up to a few times that where K is long; a limit that is set is taken as it is;
  * 0 sends every product to the tensor cores.  Both paths meet the same error bound. */
 int vtlb_set_small_gemm_limit(vtlb_ctx* ctx, double max_flops);
 

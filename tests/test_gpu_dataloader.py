@@ -151,3 +151,17 @@ def test_double_buffered_copies_overlap_compute_and_keep_order(dev):
         dev.lib.vtlb_host_free(h)
     for b in d_in + d_out:
         b.free()
+
+
+def test_batch_that_lands_in_the_dataset(sess):
+    """The caller's buffer overlaps the dataset: the rows are those before the batch was written."""
+    from vtl_b200 import host
+    x = np.arange(12 * 5, dtype=np.float32).reshape(12, 5)
+    d = sess.dev.to_device(x)
+    dl = host.DataLoader(sess, d, None, 4, True, False, 3)
+    order = dl.indices[4:8]
+    n = C.c_int(0)
+    assert dl.lib.vtlh_loader_batch(dl.h, 1, C.c_void_p(d.ptr + 2 * 5 * 4), None, C.byref(n)) == 0 and n.value == 4
+    assert np.array_equal(d.numpy()[2:6], x[order])
+    dl.close()
+    d.free()

@@ -46,3 +46,28 @@ def test_weight_gradient_into_the_weights(dev):
     assert np.allclose(dw.numpy(), g.T.astype(np.float64) @ x, rtol=1e-4, atol=1e-4)
     for b in (dg, dxin, dw, dx):
         b.free()
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 512, 600), (256, 256, 2048), (512, 64, 4096), (512, 512, 512), (33, 700, 3001)])
+def test_long_products_with_the_limit_that_nobody_set(M, N, K):
+    """Forward and backward on either side of the line between CUDA cores and tensor cores."""
+    from vtl_b200 import capi
+    dev = capi.Device(0)
+    rng = np.random.default_rng(K)
+    x, w, g = (rng.standard_normal(s).astype(np.float32) for s in ((M, K), (N, K), (M, N)))
+    d = [dev.to_device(a) for a in (x, w, g)]
+    out = [dev.to_device(np.full(s, np.nan, np.float32)) for s in ((M, N), (M, K), (N, K), (N,))]
+    dev.linear_fwd_f32(d[0], d[1], None, out[0], M, N, K)
+    dev.linear_bwd_f32(d[2], d[0], d[1], out[1], out[2], out[3], M, N, K)
+    assert dev.check_status() == 0
+    y, dx, dw, db = (o.numpy() for o in out)
+    X, W, G = (a.astype(np.float64) for a in (x, w, g))
+    # 3xTF32: 2^-22 a factor, at most 48 truncations of 2^-23 between two exact sums; f32 sums of 256 terms less
+    bound = 2 * 2.0**-22 + 48 * 2.0**-23
+    assert (np.abs(y - X @ W.T) <= bound * (np.abs(X) @ np.abs(W).T)).all()
+    assert (np.abs(dx - G @ W) <= bound * (np.abs(G) @ np.abs(W))).all()
+    assert (np.abs(dw - G.T @ X) <= bound * (np.abs(G).T @ np.abs(X))).all()
+    assert np.allclose(db, G.sum(axis=0), rtol=2.0**-23, atol=1e-12)
+    for b in d + out:
+        b.free()
+    dev.close()

@@ -76,6 +76,7 @@ struct vtlb_ctx {
   // f32 GEMMs of at most this many flops (2*M*N*K) run on the CUDA-core kernel of
   // f32_small.cu instead of the tensor-core path (vtlb_set_small_gemm_limit; 0 = never).
   double small_gemm_flops = 1.4e8;
+  bool small_gemm_default = true;  // nobody has set the limit: long products may exceed it (f32.cu, small_product)
   // Optional timing of the tensor-core GEMM launches (vtlb_profile_gemm): a ring of event
   // pairs recorded around each launch plus the algorithmic work of the launches timed.
   bool prof_on = false;

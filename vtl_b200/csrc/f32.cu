@@ -19,6 +19,8 @@ using f32::split1;
 __global__ void __launch_bounds__(256) split_rows_vec_kernel(const float4* __restrict__ src,
                                                              float4* __restrict__ hi,
                                                              float4* __restrict__ lo, size_t n4) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4;
        i += (size_t)gridDim.x * blockDim.x) {
     float4 x = src[i], h, l;
@@ -35,6 +37,8 @@ __global__ void __launch_bounds__(256) split_rows_vec_kernel(const float4* __res
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ src, int R,
                                                          int C, int ldo, float* __restrict__ hi,
                                                          float* __restrict__ lo) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const size_t n = (size_t)R * C;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -53,6 +57,8 @@ __global__ void __launch_bounds__(256) split_transpose_kernel(const float* __res
                                                               float* __restrict__ hi,
                                                               float* __restrict__ lo) {
   __shared__ float tile[32][33];
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tiles_c = (C + 31) / 32, tiles_r = (R + 31) / 32;
   const long long ntiles = (long long)tiles_c * tiles_r;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -307,6 +313,8 @@ __global__ void __launch_bounds__(128) colsum_final_kernel(const double* __restr
 __global__ void __launch_bounds__(256) colsum_short_kernel(const float* __restrict__ G, int M, int N,
                                                            float* __restrict__ out) {
   __shared__ double part[8][33];
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int n = blockIdx.x * 32 + tx;
   double s = 0.0;
@@ -360,16 +368,16 @@ int f32::split_operand(vtlb_ctx* ctx, const float* src, int rows, int kdim, bool
   if (!transposed) {
     if ((kdim & 3) == 0 && ld == kdim && vtlb_aligned16(src)) {
       const size_t n4 = (size_t)rows * kdim / 4;
-      split_rows_vec_kernel<<<f32::grid_for(ctx, n4, 256 * 4), 256, 0, ctx->stream>>>(
-          (const float4*)src, (float4*)hi, (float4*)lo, n4);
+      VTLB_CUDA(ctx, vtlb_launch_early(split_rows_vec_kernel, dim3(f32::grid_for(ctx, n4, 256 * 4)), dim3(256), 0,
+                                       ctx->stream, (const float4*)src, (float4*)hi, (float4*)lo, n4));
     } else {
-      split_rows_kernel<<<f32::grid_for(ctx, (size_t)rows * kdim, 256 * 4), 256, 0, ctx->stream>>>(
-          src, rows, kdim, ld, hi, lo);
+      VTLB_CUDA(ctx, vtlb_launch_early(split_rows_kernel, dim3(f32::grid_for(ctx, (size_t)rows * kdim, 256 * 4)), dim3(256),
+                                       0, ctx->stream, src, rows, kdim, ld, hi, lo));
     }
   } else {
     const size_t tiles = (size_t)((rows + 31) / 32) * ((kdim + 31) / 32);
-    split_transpose_kernel<<<f32::grid_for(ctx, tiles, 1), 256, 0, ctx->stream>>>(src, kdim, rows, ld,
-                                                                                 hi, lo);
+    VTLB_CUDA(ctx, vtlb_launch_early(split_transpose_kernel, dim3(f32::grid_for(ctx, tiles, 1)), dim3(256), 0, ctx->stream,
+                                     src, kdim, rows, ld, hi, lo));
   }
   VTLB_LAUNCHED(ctx);
   return VTLB_OK;
@@ -422,6 +430,26 @@ int relu_mask_inplace(vtlb_ctx* ctx, float* C, const float* mask, size_t n) {
   return vtlb_relu_bwd_f32(ctx, C, mask, C, n);
 }
 
+// Which products run on CUDA cores.  Up to the limit all; beyond it, unless the caller has set one, those whose long K
+// a tensor-core tile would walk alone: that kernel takes 14 us and 16 us per 1000 of K with its split passes, the
+// CUDA-core one 5.5 us and 85 us per GFLOP as long as its K ranges stay at 256 or less (256 x 512 x 600: 20.5 against
+// 24.8 us, 256 x 256 x 2048: 26 against 47, 512 x 64 x 4096: 28 against 80; 512 x 512 x 512: 27 against 23).
+bool ranges_short(vtlb_ctx* ctx, int M, int N, int K) {
+  return (double)((M + 31) / 32) * ((N + 63) / 64) * ((K + 255) / 256) <= 4.0 * ctx->sm_count;
+}
+bool small_product(vtlb_ctx* ctx, int M, int N, int K) {
+  const double flops = 2.0 * M * N * K;
+  if (flops <= ctx->small_gemm_flops) return true;
+  return ctx->small_gemm_default && K >= 512 && flops <= 1.0e8 + 1.9e5 * K && ranges_short(ctx, M, N, K);
+}
+// Both products of a Linear backward (contractions of N and M), which share a launch there.
+bool small_backward(vtlb_ctx* ctx, int M, int N, int K) {
+  const double flops = 2.0 * M * N * K;
+  if (flops <= ctx->small_gemm_flops) return true;
+  return ctx->small_gemm_default && flops <= 1.2e8 + 0.95e5 * ((double)M + N) && ranges_short(ctx, M, K, N) &&
+         ranges_short(ctx, N, K, M);
+}
+
 int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, const float* A,
                   const float* B, float* C, const float* bias, int relu, float* pre,
                   const GemmExtras& ex = GemmExtras()) {
@@ -430,7 +458,8 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
   const int ld_rows = vtlb_plane_ld(N), ld_cols = vtlb_plane_ld(M);
   int rc, fused = 0;
   const bool planes_in_or_out = ex.a_planes || ex.b_planes || ex.out_rows || ex.out_cols;
-  if (2.0 * M * N * K > ctx->small_gemm_flops && !planes_in_or_out && gemm2::pair_worthwhile(ctx, M, N)) {
+  const bool small = small_product(ctx, M, N, K);
+  if (!small && !planes_in_or_out && gemm2::pair_worthwhile(ctx, M, N)) {
     // Large products: f16 planes on CTA pairs, twice the tensor rate of TF32 planes and half their bytes.  Planes
     // that come in or go out are TF32 ones, so products with those keep the 3xTF32 kernel.
     const int blocks = (K + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
@@ -460,7 +489,7 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
     f32::EpiBiasRelu epi{C, bias, pre, N, relu};
     epi.mask = ex.mask;
     if ((rc = f32::launch_f16x3(ctx, p, M, N, K, epi, epoch, &fused))) return rc;
-  } else if (2.0 * M * N * K <= ctx->small_gemm_flops) {  // launch-latency-bound sizes: CUDA cores, no split passes
+  } else if (small) {  // launch-latency-bound sizes: CUDA cores, no split passes
     if ((rc = f32::sgemm_small(ctx, transA, transB, M, N, K, A, B, C, bias, relu, pre, nullptr, nullptr, ex.mask)))
       return rc;
     if (ex.mask) fused |= 2;  // the mask is part of that kernel's epilogue
@@ -511,7 +540,7 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
 int colsum(vtlb_ctx* ctx, const float* G, int M, int N, float* out) {
   vtlb_prof_scope prof(ctx, VTLB_PHASE_ELEMENTWISE);
   if (M <= 1024) {
-    colsum_short_kernel<<<(N + 31) / 32, 256, 0, ctx->stream>>>(G, M, N, out);
+    VTLB_CUDA(ctx, vtlb_launch_early(colsum_short_kernel, dim3((N + 31) / 32), dim3(256), 0, ctx->stream, G, M, N, out));
     VTLB_LAUNCHED(ctx);
     return VTLB_OK;
   }
@@ -623,7 +652,7 @@ int linear_bwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_G, const void* 
   }
   bool db_done = false;
   // a small layer: both products in one launch, where neither writes what the other reads
-  if (narrow && d_dX_or_null && d_dW_or_null && d_W && d_X && vtlb_aligned16(d_dX_or_null) && vtlb_aligned16(d_dW_or_null) &&
+  if (!any_planes && small_backward(ctx, M, N, K) && d_dX_or_null && d_dW_or_null && d_W && d_X && vtlb_aligned16(d_dX_or_null) && vtlb_aligned16(d_dW_or_null) &&
       !overlap(d_dX_or_null, (size_t)M * K, d_X, (size_t)M * K) && !overlap(d_dX_or_null, (size_t)M * K, d_G, (size_t)M * N) &&
       !overlap(d_dW_or_null, (size_t)N * K, d_W, (size_t)N * K) && !overlap(d_dW_or_null, (size_t)N * K, d_G, (size_t)M * N) &&
       !(d_relu_mask_src_or_null && overlap(d_dW_or_null, (size_t)N * K, d_relu_mask_src_or_null, (size_t)M * K)) &&
@@ -677,7 +706,7 @@ VTLB_API int vtlb_plane_ld(int kdim) { return kdim <= 0 ? 0 : (int)vtlb_round_up
 
 VTLB_API int vtlb_f32_planes_worthwhile(vtlb_ctx* ctx, int M, int N, int K) {
   // products the CUDA-core route takes never read operand planes
-  return ctx && M > 0 && N > 0 && K > 0 && 2.0 * M * N * K > ctx->small_gemm_flops;
+  return ctx && M > 0 && N > 0 && K > 0 && !small_product(ctx, M, N, K);
 }
 
 VTLB_API int vtlb_linear_fwd_f32(vtlb_ctx* ctx, const void* d_X, const void* d_W,

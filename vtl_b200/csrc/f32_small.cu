@@ -393,5 +393,6 @@ VTLB_API int vtlb_set_small_gemm_limit(vtlb_ctx* ctx, double max_flops) {
   VTLB_ENTER(ctx);
   if (max_flops < 0) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_set_small_gemm_limit: negative limit");
   ctx->small_gemm_flops = max_flops;
+  ctx->small_gemm_default = false;
   return VTLB_OK;
 }

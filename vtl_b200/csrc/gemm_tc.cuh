@@ -329,6 +329,9 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, const Epi epi, int M, int N, 
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // launched early: the set-up above overlapped the tail of the kernel in front, which is done from here on
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -572,8 +575,8 @@ int launch(vtlb_ctx* ctx, const TmapSet& tm, const Epi& epi, int M, int N, int K
   const bool timed = ctx->prof_on && ctx->prof_ev && ctx->prof_n < vtlb_ctx::kProfSlots;
   if (timed) cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n], ctx->stream);
   const int group_m = pick_group_m((M + BM - 1) / BM, (size_t)BM * K * Traits<KIND>::ELEM * Traits<KIND>::NOP);
-  kern<<<grid, NUM_THREADS, S::TOTAL, ctx->stream>>>(tm, epi, M, N, K, splits, group_m, a_chunk_k,
-                                                     ctx->d_status);
+  VTLB_CUDA(ctx, vtlb_launch_early(kern, dim3(grid), dim3(NUM_THREADS), S::TOTAL, ctx->stream, tm, epi, M, N, K, splits,
+                                   group_m, a_chunk_k, ctx->d_status));
   if (timed) {
     cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n + 1], ctx->stream);
     ctx->prof_n++;

@@ -77,16 +77,38 @@ void DataLoader::sync_indices() {
   indices_dirty_ = false;
 }
 
-Tensor DataLoader::gather(const Tensor& src, int start, int end) {
+void DataLoader::gather_into(const Tensor& src, int start, int end, float* dst) {
   Session* s = src.session();
+  const int rows = src.shape()[0];
+  s->check(vtlb_gather_rows_f32(s->ctx, src.data(), rows, src.size() / (size_t)rows,
+                                static_cast<const int*>(d_indices_->ptr) + start, end - start, dst, 0));
+}
+
+Tensor DataLoader::gather(const Tensor& src, int start, int end) {
   std::vector<int> shape = src.shape();
-  const size_t row = src.size() / (size_t)shape[0];
-  const int rows = shape[0];
   shape[0] = end - start;
-  Tensor out = Tensor::empty(s, shape);
-  s->check(vtlb_gather_rows_f32(s->ctx, src.data(), rows, row, static_cast<const int*>(d_indices_->ptr) + start,
-                                end - start, out.data(), 0));
+  Tensor out = Tensor::empty(src.session(), shape);
+  gather_into(src, start, end, out.data());
   return out;
+}
+
+int DataLoader::batch_into(int i, float* features, float* labels_out) {
+  int start, end;
+  if (!range(i, start, end)) return 0;
+  sync_indices();
+  // rows that would land in the dataset itself are gathered first and copied then
+  auto into = [&](const Tensor& src, float* dst) {
+    const size_t n = src.size() / (size_t)src.shape()[0] * (size_t)(end - start);
+    bool inside = false;
+    for (const Tensor* t : {&dataset, &labels})
+      inside = inside || (t->defined() && dst < t->data() + t->size() && t->data() < dst + n);
+    if (!inside) return gather_into(src, start, end, dst);
+    const Tensor rows = gather(src, start, end);
+    src.session()->check(vtlb_d2d(src.session()->ctx, dst, rows.data(), n * sizeof(float)));
+  };
+  into(dataset, features);
+  if (labels_out) into(labels, labels_out);
+  return end - start;
 }
 
 bool DataLoader::batch(int i, Tensor* features) {

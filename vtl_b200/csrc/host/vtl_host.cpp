@@ -210,7 +210,7 @@ struct GradBucket {
     const size_t nw = numel(wshape), nb = numel(bshape);
     const size_t off_b = (nw + 63) / 64 * 64;
     auto buf = std::make_shared<DeviceBuf>(s, (off_b + nb) * sizeof(float));
-    if (off_b != nw)  // padding travels through the all-reduce: keep it defined
+    if (s->comm_on && off_b != nw)  // padding travels through the all-reduce: keep it defined
       s->check(vtlb_memset0(s->ctx, static_cast<float*>(buf->ptr) + nw, (off_b - nw) * sizeof(float)));
     GradBucket g;
     g.dW = Tensor::view(buf, 0, wshape);

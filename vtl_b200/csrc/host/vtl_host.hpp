@@ -429,6 +429,8 @@ class DataLoader {
   DataLoader(const Tensor& dataset, const Tensor& labels /* may be undefined */, DataLoaderConfig c);
   bool batch(int i, Tensor* features);                                   // false = none (:41-84)
   bool batch_with_labels(int i, Tensor* features, Tensor* labels_out);   // (:87-143)
+  // the same into the caller's device memory; labels_out may be null; returns the number of rows, 0 = none
+  int batch_into(int i, float* features, float* labels_out);
   int len() const;                                                       // (:146-154)
   int total_samples() const { return (int)indices.size(); }
   int mini_batch_count() const { return len(); }
@@ -446,6 +448,7 @@ class DataLoader {
   bool range(int i, int& start, int& end) const;
   void sync_indices();
   Tensor gather(const Tensor& src, int start, int end);
+  void gather_into(const Tensor& src, int start, int end, float* dst);
   std::shared_ptr<DeviceBuf> d_indices_;
   bool indices_dirty_ = true;
 };

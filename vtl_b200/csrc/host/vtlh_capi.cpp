@@ -389,14 +389,9 @@ int vtlh_loader_indices(vtlh_loader* l, int* out) {
 }
 int vtlh_loader_batch(vtlh_loader* l, int i, void* d_features, void* d_labels_out, int* rows) {
   return guard([&] {
-    Tensor f, lab;
     *rows = 0;
     const bool with_labels = l->dl->labels.defined() && d_labels_out;
-    const bool ok = with_labels ? l->dl->batch_with_labels(i, &f, &lab) : l->dl->batch(i, &f);
-    if (!ok) return;
-    l->s->check(vtlb_d2d(l->s->ctx, d_features, f.data(), f.size() * sizeof(float)));
-    if (with_labels) l->s->check(vtlb_d2d(l->s->ctx, d_labels_out, lab.data(), lab.size() * sizeof(float)));
-    *rows = f.shape()[0];
+    *rows = l->dl->batch_into(i, static_cast<float*>(d_features), with_labels ? static_cast<float*>(d_labels_out) : nullptr);
   });
 }
 int vtlh_loader_split(vtlh_loader* l, double val_fraction, vtlh_loader** train, vtlh_loader** val) {
