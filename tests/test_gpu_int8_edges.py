@@ -39,6 +39,26 @@ def test_few_rows_and_their_maxima(dev, M, N, K, relu):
     _check(dev, M, N, K, relu)
 
 
+@pytest.mark.parametrize("given", [False, True])
+@pytest.mark.parametrize("M,K,offset", [(3, 1, 0), (5, 15, 0), (2, 17, 0), (7, 1023, 0), (600, 1025, 0), (4, 2047, 0),
+                                        (3, 4097, 0), (513, 8191, 0), (2, 8192, 1), (3, 1024, 2), (2, 64, 3)])
+def test_rows_that_vector_loads_cannot_take(dev, orc, M, K, offset, given):
+    A = np.random.default_rng(K).standard_normal((M, K)).astype(np.float32)
+    A[0] = 0.0
+    amax = (np.abs(A).max(axis=1) * 1.25).astype(np.float32)
+    ld = dev.i8_ld(K)
+    buf = dev.to_device(np.concatenate([np.zeros(offset, np.float32), A.ravel()]))  # a base `offset` values off
+    dM = dev.to_device(amax)
+    dQ, dS = dev.to_device(np.full((M, ld), 77, np.int8)), dev.empty((M,), np.float32)
+    dev.quant_rows_i8(buf.ptr + 4 * offset, M, K, dQ, dS, dM if given else None)
+    q_ref, s_ref = orc.quant_rows_i8_with_amax(A, amax) if given else orc.quant_rows_i8(A)
+    q = dQ.numpy()
+    assert np.array_equal(q[:, :K], q_ref) and (q[:, K:] == 77).all()
+    assert np.array_equal(dS.numpy().view(np.uint32), s_ref.view(np.uint32))
+    for b in (buf, dM, dQ, dS):
+        b.free()
+
+
 @pytest.mark.parametrize("M,K", [(1, 8208), (3, 28672), (2, 12293), (513, 8196)])
 def test_long_rows_quantised_in_pieces(dev, orc, M, K):
     A = np.random.default_rng(K).standard_normal((M, K)).astype(np.float32)
