@@ -31,7 +31,10 @@ using gemm::ROW_BYTES;
 using gemm::WAIT_LIMIT_NS;
 using igemm::Geometry;
 
-constexpr int BN = 64;
+// Columns (output channels) of a tile: 64, or 32 where there are no more.  The tensor core then fetches 11 KB of
+// operands from shared memory per 8 elements of K instead of 14, and the epilogue stages half as much: input gradient
+// of 256 x 32 x 32 x 32 -> 64, 3 x 3: 190 -> 183 us; 128 x 32 x 28 x 28 -> 32: 41.6 -> 39.4; 16 x 32 x 32 x 32: 18.8 -> 17.0.
+constexpr int MAX_BN = 64;
 constexpr int MAX_B_STAGES = 6;  // as many weight stages as the shared memory left by the staging tiles holds
 constexpr int EPI_WARPS = 4, FILL_WARPS = 8;
 constexpr int NUM_THREADS = 64 + 32 * (EPI_WARPS + FILL_WARPS);
@@ -39,8 +42,8 @@ constexpr uint32_t POLL_SLEEP_NS = 40;
 constexpr int SLAB_ROWS = 200;  // 128 positions + the largest tap shift: (kh - 1) * Wp + kw - 1 <= 72
 constexpr uint32_t SLAB_PLANE = SLAB_ROWS * ROW_BYTES;  // hi or lo part: 25 x 1024 bytes
 constexpr uint32_t SLAB = 2 * SLAB_PLANE;
-constexpr uint32_t B_TILE = BN * ROW_BYTES, B_STAGE = 2 * B_TILE;
-// Layout: two slabs | one or two staging tiles [BN channels][R * Wo pixels] f32 (output, pre-activation)
+__host__ __device__ constexpr uint32_t b_stage(int bn) { return 2u * bn * ROW_BYTES; }
+// Layout: two slabs | one or two staging tiles [32 or 64 channels][R * Wo pixels] f32 (output, pre-activation)
 // | weight stages | barriers, tensor-memory slot, tap table.
 constexpr uint32_t OUT_OFF = 2 * SLAB;
 constexpr int NUM_BARS = 2 * MAX_B_STAGES + 4 + 4 + 1;  // weights full/empty, slab full/empty, tfull/tempty, epilogue
@@ -79,11 +82,12 @@ inline bool usable(const Geometry& g, Tiling* t) {
   return true;
 }
 
-template <class Epi>
+template <int BN, class Epi>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 conv_slab_kernel(const float* __restrict__ src, const Geometry g, const Tiling tl,
                  const __grid_constant__ gemm::TmapSet tm, const Epi epi, int N, uint32_t* status) {
   constexpr int BK = 32, KSTEPS = 4, CHUNK_KB = 4;
+  constexpr uint32_t B_TILE = BN * ROW_BYTES, B_STAGE = b_stage(BN);
   // Two buffers of three accumulators each: a_hi.b_hi | a_hi.b_lo (one MMA writes both) and a_lo.b_hi.
   constexpr uint32_t ACC_COLS = 3 * BN;
   constexpr uint32_t TMEM_COLS = 512;  // 2 * ACC_COLS rounded up to a power of two
@@ -405,24 +409,24 @@ conv_slab_kernel(const float* __restrict__ src, const Geometry g, const Tiling t
 }
 
 // B planes: [N rows, ld >= K] hi and lo, k = tap * Cs + channel (regroup_weights_split_kernel)
-template <class Epi>
-int launch(vtlb_ctx* ctx, const float* src, const Geometry& g, Tiling tl, const float* b_hi, const float* b_lo,
+template <int BN, class Epi>
+int launch_bn(vtlb_ctx* ctx, const float* src, const Geometry& g, Tiling tl, const float* b_hi, const float* b_lo,
            int ldb, const Epi& epi, int N) {
   gemm::TmapSet tm;
   int rc;
   const int box_px = tl.R * g.Wo;  // a multiple of 4 pixels (16 bytes), at most 128
   tl.out_tile = (uint32_t)vtlb_round_up((size_t)BN * box_px * 4, 1024);
   tl.b_off = OUT_OFF + (epi.pre ? 2u : 1u) * tl.out_tile;
-  tl.b_stages = (int)((SMEM_MAX - 1024 - TAIL_BYTES - tl.b_off) / B_STAGE);
+  tl.b_stages = (int)((SMEM_MAX - 1024 - TAIL_BYTES - tl.b_off) / b_stage(BN));
   if (tl.b_stages > MAX_B_STAGES) tl.b_stages = MAX_B_STAGES;
-  const uint32_t smem_total = tl.b_off + tl.b_stages * B_STAGE + TAIL_BYTES + 1024;
+  const uint32_t smem_total = tl.b_off + tl.b_stages * b_stage(BN) + TAIL_BYTES + 1024;
   if ((rc = gemm::encode_tmap_3d_f32_plain(ctx, &tm.out[0], epi.Y, epi.P, epi.O, g.B, box_px, BN))) return rc;
   tm.out[1] = tm.out[0];
   if (epi.pre && (rc = gemm::encode_tmap_3d_f32_plain(ctx, &tm.out[1], epi.pre, epi.P, epi.O, g.B, box_px, BN)))
     return rc;
   if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[0], true, b_hi, g.K, N, (uint64_t)ldb * 4, 32, BN))) return rc;
   if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[1], true, b_lo, g.K, N, (uint64_t)ldb * 4, 32, BN))) return rc;
-  auto kern = conv_slab_kernel<Epi>;
+  auto kern = conv_slab_kernel<BN, Epi>;
   static std::atomic<uint64_t> configured{0};
   if (!(configured.load(std::memory_order_relaxed) >> (ctx->device & 63) & 1)) {
     VTLB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
@@ -440,6 +444,13 @@ int launch(vtlb_ctx* ctx, const float* src, const Geometry& g, Tiling tl, const 
   }
   VTLB_LAUNCHED(ctx);
   return VTLB_OK;
+}
+
+template <class Epi>
+int launch(vtlb_ctx* ctx, const float* src, const Geometry& g, const Tiling& tl, const float* b_hi, const float* b_lo,
+           int ldb, const Epi& epi, int N) {
+  return N <= 32 ? launch_bn<32, Epi>(ctx, src, g, tl, b_hi, b_lo, ldb, epi, N)
+                 : launch_bn<MAX_BN, Epi>(ctx, src, g, tl, b_hi, b_lo, ldb, epi, N);
 }
 
 }  // namespace cslab
