@@ -126,16 +126,20 @@ __global__ void __launch_bounds__(256) ckpt_decode_kernel(const unsigned char* _
       for (int g = 0; g < 8; ++g) t24[g] = b64_bits24(b64_vals4(ch[g], &bad));
     } else {  // the last group of a text, or none: 'A' (value 0) where there is no character
       const int nchar = have == 0 ? 0 : have == 1 ? 11 : 22, total = have == 0 ? 0 : have == 1 ? 12 : 24;
+      uint32_t ch[8], pad = 0;  // every character is on its way before the first is looked at
 #pragma unroll
       for (int g = 0; g < 8; ++g) {
-        uint32_t c4 = 0;
+        ch[g] = 0;
+#pragma unroll
         for (int i = 4 * g; i < 4 * g + 4; ++i) {
           const uint32_t c = i < total ? srcp[i] : '=';
-          if (i >= nchar && c != '=') atomicOr(flags, 2u);
-          c4 |= (i < nchar ? c : 'A') << (8 * (i & 3));
+          if (i >= nchar) pad |= c ^ '=';
+          ch[g] |= (i < nchar ? c : 'A') << (8 * (i & 3));
         }
-        t24[g] = b64_bits24(b64_vals4(c4, &bad));
       }
+#pragma unroll
+      for (int g = 0; g < 8; ++g) t24[g] = b64_bits24(b64_vals4(ch[g], &bad));
+      if (pad) atomicOr(flags, 2u);
     }
     double v[3];
     b64_doubles(t24, v);
