@@ -72,12 +72,15 @@ VTLB_API int vtlb_ctx_create(int device, vtlb_ctx** out) {
       (e = cudaEventCreateWithFlags(&ctx->ev_comm, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaMalloc(&ctx->d_status, 256)) != cudaSuccess ||
       (e = cudaMemset(ctx->d_status, 0, 256)) != cudaSuccess ||
+      // what the few-row kernels' row maxima need, so that calls of that size never allocate
+      (e = cudaMalloc(&ctx->scratch, (size_t)1 << 20)) != cudaSuccess ||
       (e = cudaMalloc(&ctx->ksplit_buf, vtlb_ctx::kKsplitBytes)) != cudaSuccess ||
       (e = cudaMemset(ctx->ksplit_buf, 0, vtlb_ctx::kKsplitFlagBytes)) != cudaSuccess) {
     int rc = vtlb_fail(nullptr, VTLB_ECUDA, "vtlb_ctx_create: %s", cudaGetErrorString(e));
     vtlb_ctx_destroy(ctx);
     return rc;
   }
+  ctx->scratch_bytes = (size_t)1 << 20;
   *out = ctx;
   return VTLB_OK;
 }

@@ -125,7 +125,8 @@ class Session:
         _ck(self.lib.vtlh_session_set_pass_planes(self.h, int(on)))
 
     def set_plane_min_flops(self, flops: float):
-        """Smallest product (2*M*N*K) whose planes are handed on (default 1e12)."""
+        """Smallest product (2*M*N*K) whose planes are handed on (default: none; products
+        without planes are faster)."""
         _ck(self.lib.vtlh_session_set_plane_min_flops(self.h, float(flops)))
 
     def variance_scaled(self, shape, scale, fan_mode, distribution, seed):
