@@ -551,6 +551,15 @@ int conv2d_fwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_x, const void* 
   return f32::launch_tf32x3(ctx, p, M, O, K, epi);
 }
 
+// K ranges of the lowered weight gradient, dW[O, K] over M pixels.
+int lowered_splits(vtlb_ctx* ctx, int O, int K, int M) {
+  const int mn_tiles = ((O + 127) / 128) * ((K + 63) / 64);
+  int want = (2 * ctx->sm_count + mn_tiles - 1) / mn_tiles;
+  const int max_by_len = (M + 1023) / 1024;  // at least 1024 rows of the contraction per range
+  if (want > max_by_len) want = max_by_len;
+  return f32::effective_splits(M, want);
+}
+
 int conv2d_bwd_impl(vtlb_ctx* ctx, const void* d_g, const void* d_x, const void* d_w, void* d_dx_or_null,
                     void* d_dw_or_null, void* d_db_or_null, int B, int C, int H, int W, int O, int kh, int kw, int ph,
                     int pw, int sh, int sw, int dh, int dw) {
@@ -566,6 +575,9 @@ int conv2d_bwd_impl(vtlb_ctx* ctx, const void* d_g, const void* d_x, const void*
   const bool pixel_kernel = cwgrad::usable(sh, sw, kh, kw, d.OW, dilated ? 2 : 1);
   if (d_dw_or_null && !dilated && cdirect::wgrad_worthwhile(ctx, B, C, O, d.OH, d.OW, kh, kw, pixel_kernel)) {
     if (!d_x) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_conv2d_bwd_f32: d_weight needs x");
+    // as the lowered product, which stores an uncut dW by TMA: the choice of a kernel changes nothing for the caller
+    if (!pixel_kernel && !vtlb_aligned16(d_dw_or_null) && lowered_splits(ctx, O, K, M) == 1)
+      return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_conv2d_bwd_f32: dW not 16-byte aligned");
     if ((rc = cdirect::launch_wgrad(ctx, g, (const float*)d_x, (float*)d_dw_or_null, B, C, H, W, O, d.OH, d.OW, kh, ph,
                                     pw, sh, sw)))
       return rc;
@@ -580,11 +592,7 @@ int conv2d_bwd_impl(vtlb_ctx* ctx, const void* d_g, const void* d_x, const void*
       return rc;
   } else if (d_dw_or_null) {  // dW[oc, k] = sum_m g[m, oc] * col[m, k]
     if (!d_x) return vtlb_fail(ctx, VTLB_EINVAL, "vtlb_conv2d_bwd_f32: d_weight needs x");
-    const int mn_tiles = ((O + 127) / 128) * ((K + 63) / 64);
-    int want = (2 * ctx->sm_count + mn_tiles - 1) / mn_tiles;
-    const int max_by_len = (M + 1023) / 1024;  // at least 1024 rows of the contraction per range
-    if (want > max_by_len) want = max_by_len;
-    const int S = f32::effective_splits(M, want);
+    const int S = lowered_splits(ctx, O, K, M);
     f32::Planes p;
     if ((rc = f32::alloc_planes(ctx, O, K, M, (size_t)S * O * K * sizeof(float), &p))) return rc;
     {
