@@ -61,3 +61,12 @@ def test_strided_windows(dev, B, C, H, W, O, k, pad, stride):
 @pytest.mark.parametrize("relu,bias", [(True, True), (False, False)])
 def test_small_products_on_cuda_cores(dev, B, C, H, W, O, k, pad, relu, bias):
     _check(dev, B, C, H, W, O, k, pad, 1, relu, bias)
+
+
+@pytest.mark.parametrize("B,C,H,O,k,pad", [
+    (300, 3, 8, 512, 5, 0), (300, 3, 3, 2048, 3, 0), (512, 3, 4, 512, 5, 2), (320, 64, 1, 2048, 3, 1),   # forward
+    (512, 512, 4, 3, 5, 2), (320, 2048, 1, 64, 3, 1),                                                    # input gradient
+])
+def test_many_channels_on_tiny_planes(dev, B, C, H, O, k, pad):
+    """The weights of all the channels that a CTA's threads could hold are more than a stage of shared memory."""
+    _check(dev, B, C, H, H, O, k, pad, 1)

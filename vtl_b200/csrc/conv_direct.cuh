@@ -332,15 +332,18 @@ int launch_direct_t(vtlb_ctx* ctx, Params p) {
   const long long tiles = (long long)p.B * p.tiles_y;
   p.CG = kThreads / PG < groups ? kThreads / PG : groups;
   while (p.CG > 1 && tiles * ((groups + p.CG - 1) / p.CG) < 2 * ctx->sm_count) p.CG = (p.CG + 1) / 2;
+  p.pitch = (p.W4 * PX + K - 1 + 3) / 4 * 4;
+  // One source channel has to fit the stage.  On a tiny plane a CTA could hold the weights of hundreds of channels
+  // (256 groups of 8 on one pixel group); a single group takes 4 KB at most.
+  auto channel_bytes = [&] { return ((p.TH + K - 1) * p.pitch + K * K * p.CG * CT) * 4; };
+  while (p.CG > 1 && channel_bytes() > kStageBytes) p.CG = (p.CG + 1) / 2;
+  const int per_channel = channel_bytes();
   p.Z = kThreads / (PG * p.CG);
   if (p.Z > p.Cs) p.Z = p.Cs;
   if (p.Z > 8) p.Z = 8;
-  p.pitch = (p.W4 * PX + K - 1 + 3) / 4 * 4;
-  const int per_channel = ((p.TH + K - 1) * p.pitch + K * K * p.CG * CT) * 4;
   p.CS = kStageBytes / per_channel;
   if (p.CS > p.Cs) p.CS = p.Cs;
   if (p.CS > p.Z) p.CS = p.CS / p.Z * p.Z;
-  if (p.CS < 1) p.CS = 1;
   size_t smem = (size_t)p.CS * per_channel;
   const size_t park = (size_t)(p.Z - 1) * PG * p.CG * CT * PX * 4;
   if (park > smem) smem = park;
