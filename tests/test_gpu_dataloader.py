@@ -165,3 +165,23 @@ def test_batch_that_lands_in_the_dataset(sess):
     assert np.array_equal(d.numpy()[2:6], x[order])
     dl.close()
     d.free()
+
+
+@pytest.mark.parametrize("features_at,labels_at", [("labels", None), (None, "dataset"), ("labels", "dataset")])
+def test_batch_that_lands_in_the_other_array(sess, features_at, labels_at):
+    """Features over the labels, labels over the dataset: both are rows of what was there before."""
+    from vtl_b200 import host
+    x = np.arange(12 * 5, dtype=np.float32).reshape(12, 5)
+    d, lab = sess.dev.to_device(x), sess.dev.to_device(-x)
+    spare = [sess.dev.to_device(np.zeros((4, 5), np.float32)) for _ in range(2)]
+    dl = host.DataLoader(sess, d, lab, 4, True, False, 3)
+    order = dl.indices[4:8]
+    n = C.c_int(0)
+    f = lab.ptr + 2 * 5 * 4 if features_at else spare[0].ptr
+    t = d.ptr + 3 * 5 * 4 if labels_at else spare[1].ptr
+    assert dl.lib.vtlh_loader_batch(dl.h, 1, C.c_void_p(f), C.c_void_p(t), C.byref(n)) == 0 and n.value == 4
+    assert np.array_equal(lab.numpy()[2:6] if features_at else spare[0].numpy(), x[order])
+    assert np.array_equal(d.numpy()[3:7] if labels_at else spare[1].numpy(), -x[order])
+    dl.close()
+    for b in (d, lab, *spare):
+        b.free()

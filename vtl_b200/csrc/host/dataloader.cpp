@@ -96,18 +96,24 @@ int DataLoader::batch_into(int i, float* features, float* labels_out) {
   int start, end;
   if (!range(i, start, end)) return 0;
   sync_indices();
-  // rows that would land in the dataset itself are gathered first and copied then
-  auto into = [&](const Tensor& src, float* dst) {
-    const size_t n = src.size() / (size_t)src.shape()[0] * (size_t)(end - start);
-    bool inside = false;
+  auto count = [&](const Tensor& src) { return src.size() / (size_t)src.shape()[0] * (size_t)(end - start); };
+  auto inside = [&](const float* dst, size_t n) {  // the dataset or the labels
+    bool in = false;
     for (const Tensor* t : {&dataset, &labels})
-      inside = inside || (t->defined() && dst < t->data() + t->size() && t->data() < dst + n);
-    if (!inside) return gather_into(src, start, end, dst);
-    const Tensor rows = gather(src, start, end);
-    src.session()->check(vtlb_d2d(src.session()->ctx, dst, rows.data(), n * sizeof(float)));
+      in = in || (t->defined() && dst < t->data() + t->size() && t->data() < dst + n);
+    return in;
   };
-  into(dataset, features);
-  if (labels_out) into(labels, labels_out);
+  if (inside(features, count(dataset)) || (labels_out && inside(labels_out, count(labels)))) {
+    // every row is read before the first is written
+    Session* s = dataset.session();
+    const Tensor f = gather(dataset, start, end);
+    const Tensor l = labels_out ? gather(labels, start, end) : Tensor();
+    s->check(vtlb_d2d(s->ctx, features, f.data(), f.size() * sizeof(float)));
+    if (labels_out) s->check(vtlb_d2d(s->ctx, labels_out, l.data(), l.size() * sizeof(float)));
+  } else {
+    gather_into(dataset, start, end, features);
+    if (labels_out) gather_into(labels, start, end, labels_out);
+  }
   return end - start;
 }
 
