@@ -102,3 +102,19 @@ def test_linear_backward(dev, wide):
     assert (np.abs(db - ref) <= 2.0**-24 * np.abs(ref) + 1e-13 * np.abs(g).sum(axis=0)).all()
     for b in d + out:
         b.free()
+
+
+def test_scratch_of_a_large_product():
+    """The context keeps the operands' planes, 8 bytes an element, and little beside them."""
+    from vtl_b200.capi import Device
+    dev = Device(0)
+    M, N, K = 8192, 4096, 4096
+    bufs = [dev.to_device(np.zeros(s, np.float32)) for s in ((M, K), (N, K), (M, N))]
+    dev.sync()
+    free = torch.cuda.mem_get_info()[0]
+    dev.gemm_f32(False, True, M, N, K, *bufs)
+    dev.sync()
+    assert free - torch.cuda.mem_get_info()[0] < 1.25 * 8 * (M + N) * K
+    for b in bufs:
+        b.free()
+    dev.close()

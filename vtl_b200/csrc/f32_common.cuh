@@ -70,9 +70,9 @@ inline int alloc_half_planes(vtlb_ctx* ctx, int rows_a, int rows_b, int K, size_
   p->lda_scale = (int)vtlb_round_up((size_t)rows_a, 256);
   p->ldb_scale = (int)vtlb_round_up((size_t)rows_b, 256) / gemm::kHalfGroup;
   const size_t a = vtlb_round_up((size_t)rows_a * p->ld, 128), b = vtlb_round_up((size_t)rows_b * p->ld, 128);
-  const size_t front = (2 * a + 2 * b) * sizeof(__half);
   const size_t sa = blocks * p->lda_scale, sb = vtlb_round_up(blocks * p->ldb_scale, 64);
-  if (int rc = alloc_planes(ctx, rows_a, rows_b, K, front + (sa + sb) * sizeof(float) + extra_bytes, &p->tf32)) return rc;
+  if (int rc = alloc_planes(ctx, rows_a, rows_b, K, (sa + sb) * sizeof(float) + extra_bytes, &p->tf32)) return rc;
+  // a pair of f16 planes takes no more than the pair of TF32 planes in whose place it lies: ld is at most twice theirs
   p->a_hi = (__half*)p->tf32.a_hi;
   p->a_lo = p->a_hi + a;
   p->b_hi = p->a_lo + a;
