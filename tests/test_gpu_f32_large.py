@@ -70,6 +70,74 @@ def test_operands_of_any_range(dev, kind):
     assert _error(_product(dev, False, True, A, B), A, B) < 2 * 2.0**-22 + 48 * 2.0**-23
 
 
+LIMIT = 2 * 2.0**-22 + 48 * 2.0**-23  # 3xTF32's, element by element
+
+
+def _pruned(rng, r, K, every, scale=None):
+    """Normal values in every `every`-th column: alone there, or `scale` times smaller than the others."""
+    x, some = rng.standard_normal((r, K)), np.arange(K) % every == every // 2
+    return (x * some if scale is None else np.where(some, x * scale, x)).astype(np.float32)
+
+
+@pytest.mark.parametrize("ta,tb", [(False, True), (True, False)])
+@pytest.mark.parametrize("s", [1e-4, 1e-6, 1e-7, 1e-9, 1e-11, 1e-13, 1e-30])
+def test_small_elements_that_meet_the_only_large_ones(dev, s, ta, tb):
+    """The elements of one operand that f16 cannot hold beside their neighbours are the ones that count: the other
+    operand is zero wherever this one is large."""
+    M, N, K = 1536, 1792, 600
+    rng = np.random.default_rng(6)
+    A, B = _pruned(rng, M, K, 20, s), _pruned(rng, N, K, 20)
+    assert _error(_product(dev, ta, tb, A, B), A, B) < LIMIT
+    A, B = _pruned(rng, M, K, 20), _pruned(rng, N, K, 20, s)
+    assert _error(_product(dev, ta, tb, A, B), A, B) < LIMIT
+
+
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("few", [1, 3, 4, 5, 6, 60])
+def test_few_small_elements(dev, ta, tb, few):
+    """So few that the product stays on f16 planes (5 in one row of a block, or 60 in all, are too many): planted in both
+    operands, at the edges of blocks, groups and the matrices, some of them opposite one another."""
+    M, N, K = 1501, 1797, 775
+    rng = np.random.default_rng(few)
+    A, B = rng.standard_normal((M, K)), rng.standard_normal((N, K))
+    ks = np.array([0, 255, 256, 511, 512, 767, 768, 774, 300, 301])
+    if few <= 5:  # in one row of one block
+        A[5, 256:256 + few] *= 10.0 ** -np.arange(10, 10 + few)
+        B[M % 31, 512:512 + few] *= 10.0 ** -np.arange(10, 10 + few)
+        B[:, 256:256 + few] *= 1e3
+        A[:, 512:512 + few] *= 1e3
+    else:
+        rows, cols = rng.choice(M, few, replace=False), rng.choice(N, few, replace=False)
+        rows[:3], cols[:3] = (0, 31, M - 1), (0, 32, N - 1)
+        A[rows, ks[np.arange(few) % 10]] *= 10.0 ** -rng.uniform(9, 18, few)
+        B[cols, ks[np.arange(few) % 10]] *= 10.0 ** -rng.uniform(9, 18, few)
+        keep = np.zeros(K, bool)  # and nothing else meets them
+        keep[ks] = True
+        B[:N // 2, ~keep] = 0
+        A[M // 2:, ~keep] = 0
+    A, B = A.astype(np.float32), B.astype(np.float32)
+    assert _error(_product(dev, ta, tb, A, B), A, B) < LIMIT
+
+
+@pytest.mark.parametrize("tb", [False, True])
+@pytest.mark.parametrize("kind", ["diagonal", "permutation", "sparse"])
+def test_sparse_second_operand(dev, kind, tb):
+    """32 rows of B share a scale: a row of a single value has to survive beside much larger ones."""
+    M, N, K = 1536, 1792, 512
+    rng = np.random.default_rng(7)
+    A, B = rng.standard_normal((M, K)), np.zeros((N, K))
+    at = rng.permutation(K)
+    if kind == "diagonal":
+        B[at, np.arange(K)] = 10.0 ** -np.linspace(0, 12, K)[rng.permutation(K)]
+    if kind == "permutation":
+        A *= 10.0 ** rng.uniform(-9, 0, A.shape)
+        B[at, np.arange(K)] = 1
+    if kind == "sparse":
+        B = rng.standard_normal((N, K)) * (rng.random((N, K)) < 0.005) * 10.0 ** rng.uniform(-9, 0, (N, K))
+    A, B = A.astype(np.float32), B.astype(np.float32)
+    assert _error(_product(dev, False, tb, A, B), A, B) < LIMIT
+
+
 def test_infinities_and_nans_stay_in_their_rows(dev):
     M, N, K = 1536, 1792, 512
     rng = np.random.default_rng(4)

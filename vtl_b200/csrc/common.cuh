@@ -31,10 +31,11 @@ struct vtlb_ctx {
   // next batch comes in and the last result goes out while the current step computes
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
   cudaEvent_t ev_copy = nullptr;       // ordering between the copy streams and compute
-  // device status word, (kTicketWord) the block ticket of last_block() and (kUnfitWord) the epoch of the last
-  // f32 product whose operands did not fit f16 planes
+  // device status word, (kTicketWord) the block ticket of last_block(), and of f32 products on f16 planes the epoch of
+  // the last one whose operands did not fit (kUnfitWord), of the last one with elements to be multiplied by themselves
+  // (kListedWord) and how many such the operands of the one under way have (kRestWord, two words)
   uint32_t* d_status = nullptr;
-  static constexpr int kTicketWord = 32, kUnfitWord = 40;
+  static constexpr int kTicketWord = 32, kUnfitWord = 40, kListedWord = 41, kRestWord = 48;
   uint32_t half_epoch = 0;             // products on f16 planes so far, never 0
   void* scratch = nullptr;             // operand-split buffers, partial sums
   size_t scratch_bytes = 0;

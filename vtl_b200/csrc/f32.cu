@@ -92,10 +92,6 @@ __device__ __forceinline__ void block_scale(float amax, float& mul, float& inv) 
   mul = __uint_as_float((uint32_t)(127 + e) << 23);
   inv = __uint_as_float((uint32_t)(127 - e) << 23);
 }
-__device__ __forceinline__ void split_half(float x, __half& hi, __half& lo) {
-  hi = __float2half_rn(x);
-  lo = __float2half_rn(x - __half2float(hi));
-}
 __device__ __forceinline__ float warp_amax(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -112,30 +108,71 @@ __device__ __forceinline__ float block_amax(float v, float (&part)[8]) {
   for (int w = 1; w < 8; ++w) v = fmaxf(v, part[w]);
   return v;
 }
-// Says that f16 cannot hold a block of 256 values, eight per lane, as well as TF32 does (struct HalfPlanes): more
-// than one in sixteen of those that are not zero (and more than a stray one) scaled below 2^-4, or a scale so
-// extreme that the product of two such would leave the f32 range (an infinity in the block among them).
-__device__ __forceinline__ void note_unfit(const float (&v)[8], float mul, uint32_t* unfit, uint32_t epoch) {
-  uint32_t n = 0;
+// Where a split pass puts the planes of an operand and what belongs to them (gemm::HalfSide), and how it says that f16
+// cannot hold the operand: elements listed so far and how many may be, the word and the product's epoch.
+struct HalfOut {
+  __half *hi, *lo;
+  float* scale;
+  uint8_t* flags;
+  int2* rest;
+  int ld, rp;
+  uint32_t *count, *unfit, *listed;
+  uint32_t limit, epoch;
+};
+// One scale of a block: so extreme that the product of two such would leave the f32 range (an infinity in the block
+// among them)?
+__device__ __forceinline__ void note_scale(float mul, const HalfOut& o) {
+  if (mul > 0x1p74f || mul < 0x1p-63f) *o.unfit = o.epoch;
+}
+constexpr float kHalfUp = (float)(1 << gemm::kHalfShift), kHalfDown = 1.0f / kHalfUp;
+// x in two halves of the scaled value; true if they do not hold it to 22 bits.  hi + lo / 2^12 is exact in f32 (a
+// multiple of the scaled value's last bit and no longer than it), and so is what is left of x.
+__device__ __forceinline__ float half_rest(float x, float inv, __half hi, __half lo) {
+  return __fmaf_rn(-__fmaf_rn(__half2float(lo), kHalfDown, __half2float(hi)), inv, x);
+}
+__device__ __forceinline__ bool split_half(float x, float mul, float inv, __half& hi, __half& lo) {
+  const float v = x * mul;
+  hi = __float2half_rn(v);
+  lo = __float2half_rn((v - __half2float(hi)) * kHalfUp);
+  return fabsf(half_rest(x, inv, hi, lo)) > 0x1p-22f * fabsf(x);
+}
+// Lists what the halves of one row's block leave, eight elements per lane: bit j of `bad` (of some lane) says that
+// element j, at k_of(j), is not held.  In the order of the lanes, so that a run repeats itself.
+template <class KOf>
+__device__ __forceinline__ void list_rests(uint32_t bad, const float (&x)[8], float mul, float inv, KOf k_of, int kb,
+                                           int row, const HalfOut& o) {
+  const int lane = threadIdx.x & 31;
+  int at = __popc(bad);
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int before = __shfl_up_sync(0xffffffffu, at, d);
+    if (lane >= d) at += before;
+  }
+  const int n = __shfl_sync(0xffffffffu, at, 31);
+  at -= __popc(bad);
+  int2* list = o.rest + ((size_t)kb * o.rp + row) * gemm::kHalfRest;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float a = fabsf(v[j]);
-    n += (a > 0.0f ? 1u : 0u) + (a > 0.0f && a * mul < 0.0625f ? 0x10000u : 0u);
+    if (bad >> j & 1u) {
+      __half hi, lo;
+      split_half(x[j], mul, inv, hi, lo);
+      if (at < gemm::kHalfRest) list[at] = make_int2(k_of(j), __float_as_int(half_rest(x[j], inv, hi, lo)));
+      ++at;
+    }
   }
-  n = __reduce_add_sync(0xffffffffu, n);
-  const uint32_t small = n >> 16, nonzero = n & 0xffffu;
-  const bool extreme = mul > 1.8889466e22f || mul < 1.0842022e-19f;  // 2^74, 2^-63
-  if ((threadIdx.x & 31) == 0 && (extreme || (small >= 2 && small * 16 > nonzero))) *unfit = epoch;
+  if (lane >= n && lane < gemm::kHalfRest) list[lane] = make_int2(-1, 0);
+  if (lane == 0) {
+    *o.listed = o.epoch;
+    if (n > gemm::kHalfRest || atomicAdd(o.count, (uint32_t)n) + n > o.limit) *o.unfit = o.epoch;
+  }
 }
 
-// src [R, C] row-major -> scaled f16 planes [R, ld] and factors.  A CTA takes 32 rows x 256 values, a warp four of
-// the rows, eight values per lane.  GROUP: one scale for the 32 rows (operand B), else one per row.
+// src [R, C] row-major -> scaled f16 planes [R, ld] and what belongs to them.  A CTA takes 32 rows x 256 values, a warp
+// four of the rows, eight values per lane.  GROUP: one scale for the 32 rows (operand B), else one per row.
 // Bound by HBM, 8 bytes per element: 8192 x 4096 in 43 us (6.2 TB/s); the TF32 planes, 12 bytes, took 70 us.
 template <bool VEC, bool GROUP>
-__global__ void __launch_bounds__(256) split_rows_half_kernel(const float* __restrict__ src, int R, int C, int ld,
-                                                              int lds, __half* __restrict__ hi,
-                                                              __half* __restrict__ lo, float* __restrict__ scale,
-                                                              uint32_t* unfit, uint32_t epoch) {
+__global__ void __launch_bounds__(256) split_rows_half_kernel(const float* __restrict__ src, int R, int C,
+                                                              const HalfOut o) {
   __shared__ float part[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int blocks = (C + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
@@ -167,35 +204,51 @@ __global__ void __launch_bounds__(256) split_rows_half_kernel(const float* __res
       all = fmaxf(all, m[q]);
     }
     if (GROUP) all = block_amax(all, part);
+    uint32_t bad = 0;  // bit 8 q + j: element j of row q is not held
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       float mul, inv;
       block_scale(GROUP ? all : warp_amax(m[q]), mul, inv);
-      note_unfit(v[q], mul, unfit, epoch);
       if (r0 + q >= R) break;
+      if (lane == 0 && (!GROUP || q == 0)) note_scale(mul, o);
       union { __half h[8]; uint4 u; } ph, pl;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) split_half(v[q][j] * mul, ph.h[j], pl.h[j]);
-      if (c < ld) {  // ld is C rounded up to 8
-        *reinterpret_cast<uint4*>(hi + (size_t)(r0 + q) * ld + c) = ph.u;
-        *reinterpret_cast<uint4*>(lo + (size_t)(r0 + q) * ld + c) = pl.u;
+      for (int j = 0; j < 8; ++j) bad |= split_half(v[q][j], mul, inv, ph.h[j], pl.h[j]) ? 1u << (8 * q + j) : 0u;
+      if (c < o.ld) {  // ld is C rounded up to 8
+        *reinterpret_cast<uint4*>(o.hi + (size_t)(r0 + q) * o.ld + c) = ph.u;
+        *reinterpret_cast<uint4*>(o.lo + (size_t)(r0 + q) * o.ld + c) = pl.u;
       }
-      if (!GROUP && lane == 0) scale[(size_t)kb * lds + r0 + q] = inv;
-      if (GROUP && threadIdx.x == 0 && q == 0) scale[(size_t)kb * lds + grp] = inv;
+      if (!GROUP && lane == 0) o.scale[(size_t)kb * o.rp + r0 + q] = inv;
+      if (GROUP && threadIdx.x == 0 && q == 0) o.scale[(size_t)kb * (o.rp / gemm::kHalfGroup) + grp] = inv;
     }
+    uint32_t flags = 0;
+    if (__any_sync(0xffffffffu, bad != 0)) {  // seldom: the row is read again, which leaves the registers to the rest
+#pragma unroll 1
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t b = bad >> (8 * q) & 0xffu;
+        if (!__any_sync(0xffffffffu, b != 0)) continue;
+        float x[8], mx = 0.0f, mul, inv;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          x[j] = c + j < C ? __ldg(src + (size_t)(r0 + q) * C + c + j) : 0.0f;
+          mx = fmaxf(mx, fabsf(x[j]));
+        }
+        block_scale(GROUP ? all : warp_amax(mx), mul, inv);
+        list_rests(b, x, mul, inv, [&](int j) { return c + j; }, kb, r0 + q, o);
+        flags |= 1u << q;
+      }
+    }
+    if (lane == 0) o.flags[(size_t)kb * (o.rp / 4) + r0 / 4] = (uint8_t)flags;
   }
 }
 
-// src [R, C] row-major -> planes of the transpose, [C, ld >= R], and factors; where `colsum` is given, also the f64
-// column sums of each block, colsum[block][C] (the bias gradient's partial sums: a pass of its own over the gradient
-// took 71 us per 8192 x 4096).  A CTA turns 256 rows x 32 columns through shared memory: 128-byte rows in, and a
-// warp writes 128 contiguous bytes of a plane per instruction.  8192 x 4096: 57 us (73 us for TF32 planes).
+// src [R, C] row-major -> planes of the transpose, [C, ld >= R], and what belongs to them; where `colsum` is given, also
+// the f64 column sums of each block, colsum[block][C] (the bias gradient's partial sums: a pass of its own over the
+// gradient took 71 us per 8192 x 4096).  A CTA turns 256 rows x 32 columns through shared memory: 128-byte rows in, and
+// a warp writes 128 contiguous bytes of a plane per instruction.  8192 x 4096: 57 us (73 us for TF32 planes).
 template <bool GROUP>
-__global__ void __launch_bounds__(256) split_transpose_half_kernel(const float* __restrict__ src, int R, int C, int ld,
-                                                                   int lds, __half* __restrict__ hi,
-                                                                   __half* __restrict__ lo, float* __restrict__ scale,
-                                                                   double* __restrict__ colsum, uint32_t* unfit,
-                                                                   uint32_t epoch) {
+__global__ void __launch_bounds__(256) split_transpose_half_kernel(const float* __restrict__ src, int R, int C,
+                                                                   double* __restrict__ colsum, const HalfOut o) {
   __shared__ float tile[gemm::kHalfBlock][33];
   __shared__ float part[8];
   const int tiles_c = (C + 31) / 32, tiles_r = (R + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
@@ -215,6 +268,7 @@ __global__ void __launch_bounds__(256) split_transpose_half_kernel(const float* 
     }
     if (GROUP) all = block_amax(all, part);
     else __syncthreads();
+    uint32_t bad = 0;  // bit 8 q + j: element j of column q is not held
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int col = warp * 4 + q, cg = c0 + col;
@@ -228,29 +282,47 @@ __global__ void __launch_bounds__(256) split_transpose_half_kernel(const float* 
         m = fmaxf(m, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
       }
       block_scale(GROUP ? all : warp_amax(m), mul, inv);
-      note_unfit(v, mul, unfit, epoch);
+      if (lane == 0 && (!GROUP || q == 0)) note_scale(mul, o);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = r0 + i * 64 + lane * 2;
-        if (r < ld) {  // ld is R rounded up to 8
-          __half2 h, l;
-          split_half(v[2 * i] * mul, h.x, l.x);
-          split_half(v[2 * i + 1] * mul, h.y, l.y);
-          *reinterpret_cast<__half2*>(hi + (size_t)cg * ld + r) = h;
-          *reinterpret_cast<__half2*>(lo + (size_t)cg * ld + r) = l;
+        __half2 h, l;
+        bad |= split_half(v[2 * i], mul, inv, h.x, l.x) ? 1u << (8 * q + 2 * i) : 0u;
+        bad |= split_half(v[2 * i + 1], mul, inv, h.y, l.y) ? 2u << (8 * q + 2 * i) : 0u;
+        if (r < o.ld) {  // ld is R rounded up to 8
+          *reinterpret_cast<__half2*>(o.hi + (size_t)cg * o.ld + r) = h;
+          *reinterpret_cast<__half2*>(o.lo + (size_t)cg * o.ld + r) = l;
         }
       }
-      if (!GROUP && lane == 0) scale[(size_t)kb * lds + cg] = inv;
-      if (GROUP && threadIdx.x == 0 && q == 0) scale[(size_t)kb * lds + c0 / 32] = inv;
+      if (!GROUP && lane == 0) o.scale[(size_t)kb * o.rp + cg] = inv;
+      if (GROUP && threadIdx.x == 0 && q == 0) o.scale[(size_t)kb * (o.rp / gemm::kHalfGroup) + c0 / 32] = inv;
       if (colsum) {
         double s = 0.0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) s = __dadd_rn(s, (double)v[i]);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        for (int o2 = 16; o2 > 0; o2 >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o2));
         if (lane == 0) colsum[(size_t)kb * C + cg] = s;
       }
     }
+    uint32_t flags = 0;
+    if (__any_sync(0xffffffffu, bad != 0)) {  // seldom
+#pragma unroll 1
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t b = bad >> (8 * q) & 0xffu;
+        if (!__any_sync(0xffffffffu, b != 0)) continue;
+        float x[8], mx = 0.0f, mul, inv;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          x[j] = tile[(j >> 1) * 64 + lane * 2 + (j & 1)][warp * 4 + q];
+          mx = fmaxf(mx, fabsf(x[j]));
+        }
+        block_scale(GROUP ? all : warp_amax(mx), mul, inv);
+        list_rests(b, x, mul, inv, [&](int j) { return r0 + (j >> 1) * 64 + lane * 2 + (j & 1); }, kb, c0 + warp * 4 + q, o);
+        flags |= 1u << q;
+      }
+    }
+    if (lane == 0) o.flags[(size_t)kb * (o.rp / 4) + c0 / 4 + warp] = (uint8_t)flags;
   }
 }
 
@@ -261,8 +333,9 @@ struct SplitSource {
   int rows, kdim, ld, transposed;  // transposed: stored [kdim, rows]
 };
 __global__ void __launch_bounds__(256) split_unfit_kernel(SplitSource a, SplitSource b, const uint32_t* unfit,
-                                                          uint32_t epoch) {
+                                                          uint32_t epoch, uint32_t* counts) {
   __shared__ float tile[32][33];
+  if (blockIdx.x == 0 && threadIdx.x < 2) counts[threadIdx.x] = 0;  // listed elements: the next product counts again
   if (*unfit != epoch) return;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int o = 0; o < 2; ++o) {
@@ -408,19 +481,24 @@ struct GemmExtras {
 
 // Splits one operand into f16 planes; `transposed` says src is stored [kdim, rows], `group` that 32 rows share a
 // scale (operand B).
-int split_operand_half(vtlb_ctx* ctx, const float* src, int rows, int kdim, bool transposed, bool group, int ld, int lds,
-                       __half* hi, __half* lo, float* scale, double* colsum, uint32_t epoch) {
+int split_operand_half(vtlb_ctx* ctx, const float* src, int kdim, bool transposed, bool group, int ld,
+                       const f32::HalfPlanes::Side& p, double* colsum, uint32_t epoch) {
   vtlb_prof_scope prof(ctx, VTLB_PHASE_SPLIT);
-  uint32_t* unfit = ctx->d_status + vtlb_ctx::kUnfitWord;
-  const int grid = f32::grid_for(ctx, (size_t)((rows + 31) / 32) * ((kdim + gemm::kHalfBlock - 1) / gemm::kHalfBlock), 1);
+  HalfOut o{p.hi, p.lo, p.scale, p.flags, p.rest, ld, p.rp};
+  o.count = ctx->d_status + vtlb_ctx::kRestWord + (group ? 1 : 0);
+  o.unfit = ctx->d_status + vtlb_ctx::kUnfitWord;
+  o.listed = ctx->d_status + vtlb_ctx::kListedWord;
+  o.limit = 4u + (uint32_t)((unsigned long long)p.rows * kdim >> 19);
+  o.epoch = epoch;
+  const int grid = f32::grid_for(ctx, (size_t)((p.rows + 31) / 32) * ((kdim + gemm::kHalfBlock - 1) / gemm::kHalfBlock), 1);
   if (transposed) {
     auto kern = group ? split_transpose_half_kernel<true> : split_transpose_half_kernel<false>;
-    kern<<<grid, 256, 0, ctx->stream>>>(src, kdim, rows, ld, lds, hi, lo, scale, colsum, unfit, epoch);
+    kern<<<grid, 256, 0, ctx->stream>>>(src, kdim, p.rows, colsum, o);
   } else {
     const bool vec = (kdim & 3) == 0 && vtlb_aligned16(src);
     auto kern = group ? (vec ? split_rows_half_kernel<true, true> : split_rows_half_kernel<false, true>)
                       : (vec ? split_rows_half_kernel<true, false> : split_rows_half_kernel<false, false>);
-    kern<<<grid, 256, 0, ctx->stream>>>(src, rows, kdim, ld, lds, hi, lo, scale, unfit, epoch);
+    kern<<<grid, 256, 0, ctx->stream>>>(src, p.rows, kdim, o);
   }
   VTLB_LAUNCHED(ctx);
   return VTLB_OK;
@@ -465,16 +543,12 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
     const int blocks = (K + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
     const bool sums = ex.a_colsum && transA;
     f32::HalfPlanes p;
-    if ((rc = f32::alloc_half_planes(ctx, M, N, K, sums ? (size_t)blocks * M * sizeof(double) + 256 : 0, &p))) return rc;
-    double* partial = sums ? (double*)vtlb_round_up((size_t)p.extra, 256) : nullptr;
+    if ((rc = f32::alloc_half_planes(ctx, M, N, K, sums ? (size_t)blocks * M * sizeof(double) : 0, &p))) return rc;
+    double* partial = sums ? (double*)p.extra : nullptr;
     if (++ctx->half_epoch == 0) ctx->half_epoch = 1;
     const uint32_t epoch = ctx->half_epoch;
-    if ((rc = split_operand_half(ctx, A, M, K, transA != 0, false, p.ld, p.lda_scale, p.a_hi, p.a_lo, p.a_scale, partial,
-                                 epoch)))
-      return rc;
-    if ((rc = split_operand_half(ctx, B, N, K, transB == 0, true, p.ld, p.ldb_scale, p.b_hi, p.b_lo, p.b_scale, nullptr,
-                                 epoch)))
-      return rc;
+    if ((rc = split_operand_half(ctx, A, K, transA != 0, false, p.ld, p.a, partial, epoch))) return rc;
+    if ((rc = split_operand_half(ctx, B, K, transB == 0, true, p.ld, p.b, nullptr, epoch))) return rc;
     if (sums) {
       colsum_final_kernel<<<(M + 127) / 128, 128, 0, ctx->stream>>>(partial, blocks, M, ex.a_colsum);
       VTLB_LAUNCHED(ctx);
@@ -483,7 +557,8 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
     {
       const SplitSource sa{A, p.tf32.a_hi, p.tf32.a_lo, M, K, p.tf32.ld, transA != 0};
       const SplitSource sb{B, p.tf32.b_hi, p.tf32.b_lo, N, K, p.tf32.ld, transB == 0};
-      split_unfit_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(sa, sb, ctx->d_status + vtlb_ctx::kUnfitWord, epoch);
+      split_unfit_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(sa, sb, ctx->d_status + vtlb_ctx::kUnfitWord, epoch,
+                                                                     ctx->d_status + vtlb_ctx::kRestWord);
       VTLB_LAUNCHED(ctx);
     }
     f32::EpiBiasRelu epi{C, bias, pre, N, relu};

@@ -1,7 +1,6 @@
 // Pieces shared by the f32 GEMM users (f32.cu, conv.cu): the TF32 hi/lo split, the
 // operand planes in the context scratch, and the launcher of the 3xTF32 tcgen05 GEMM.
 #pragma once
-#include <cuda_fp16.h>
 #include <stdlib.h>
 
 #include "gemm_tc2.cuh"
@@ -49,38 +48,61 @@ inline int alloc_planes(vtlb_ctx* ctx, int rows_a, int rows_b, int K, size_t ext
 
 // Two K-major operands, each as a pair of f16 planes [rows, ld] of scaled values: a block of 256 elements along K
 // of a row of A (of 32 rows of B) is multiplied by the power of two that brings its largest into [2^14, 2^15), and
-//     x * 2^e = hi + lo,  hi = f16(x * 2^e), lo = f16(x * 2^e - hi).
+//     x * 2^e = hi + lo / 2^12,  hi = f16(x * 2^e), lo = f16((x * 2^e - hi) * 2^12).
 // hi and lo have 11 significant bits each, as TF32 has, so the three products lo.hi + hi.lo + hi.hi lose what the
-// 3xTF32 ones lose, 2^-22 of a term.  Where lo is below f16's normal range, an element keeps 2^-25 of its scaled
-// value instead: that is as good down to 2^-4 = 2^-18 of its block's largest.  The split passes count the elements
-// below that; a block with more than one in sixteen of them (features on very different scales, say) makes the
-// operands unfit, and the product runs on TF32 planes after all, from a launch behind this one that otherwise
-// returns at once.  The TF32 planes take the f16 ones' place in scratch.
+// 3xTF32 ones lose, 2^-22 of a term.  lo's factor, which the tensor core takes back for nothing, puts it far into f16's
+// normal range: an element keeps 22 bits down to 2^-15, 2^-29 of its block's largest (without it to 2^-17), and below
+// that an error of 2^-37 of the scaled value.  No bound on the sum makes up for that: the other operand may be zero
+// wherever this one is large.  What the planes leave of such an element is therefore listed (gemm::HalfSide::rest) and
+// multiplied in f32 by the kernel's epilogue.  Of 33 M normally distributed elements one in thirty operands has any.
+// Each costs a warp 5 us in every tile of its row (loads beside the operands' stream), so with more than 4 + one in 2^19,
+// which one warp may have all of, 3xTF32 would be faster; with those, or more than kHalfRest in one row of a block, the
+// operands are unfit and the product runs on TF32 planes after all, from
+// a launch behind this one that otherwise returns at once.  The TF32 planes take the f16 ones' place in scratch.
 struct HalfPlanes {
-  __half *a_hi, *a_lo, *b_hi, *b_lo;
-  float *a_scale, *b_scale;  // 2^-e, [blocks of K][rows of A / groups of B, padded to whole tiles]
-  int ld;                    // row stride in elements: K rounded up to 8 (TMA wants 16-byte strides)
-  int lda_scale, ldb_scale;
+  struct Side {
+    __half *hi, *lo;
+    float* scale;
+    uint8_t* flags;
+    int2* rest;
+    int rows, rp;  // rp: rows rounded up to whole tiles
+  } a, b;
+  int ld;          // row stride in elements: K rounded up to 8 (TMA wants 16-byte strides)
   Planes tf32;
-  void* extra;
+  void* extra;     // `extra_bytes` of additional scratch, 256-byte aligned
 };
 inline int alloc_half_planes(vtlb_ctx* ctx, int rows_a, int rows_b, int K, size_t extra_bytes, HalfPlanes* p) {
   p->ld = (int)vtlb_round_up((size_t)K, 8);
   const size_t blocks = (size_t)(K + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
-  p->lda_scale = (int)vtlb_round_up((size_t)rows_a, 256);
-  p->ldb_scale = (int)vtlb_round_up((size_t)rows_b, 256) / gemm::kHalfGroup;
-  const size_t a = vtlb_round_up((size_t)rows_a * p->ld, 128), b = vtlb_round_up((size_t)rows_b * p->ld, 128);
-  const size_t sa = blocks * p->lda_scale, sb = vtlb_round_up(blocks * p->ldb_scale, 64);
-  if (int rc = alloc_planes(ctx, rows_a, rows_b, K, (sa + sb) * sizeof(float) + extra_bytes, &p->tf32)) return rc;
-  // a pair of f16 planes takes no more than the pair of TF32 planes in whose place it lies: ld is at most twice theirs
-  p->a_hi = (__half*)p->tf32.a_hi;
-  p->a_lo = p->a_hi + a;
-  p->b_hi = p->a_lo + a;
-  p->b_lo = p->b_hi + b;
-  // the factors lie behind both kinds of planes
-  p->a_scale = (float*)p->tf32.extra;
-  p->b_scale = p->a_scale + sa;
-  p->extra = p->b_scale + sb;
+  HalfPlanes::Side* side[2] = {&p->a, &p->b};
+  size_t behind = 256;  // bytes behind the planes; pieces start on 256-byte boundaries
+  auto piece = [&](size_t bytes) {
+    const size_t at = behind;
+    behind += vtlb_round_up(bytes, 256);
+    return at;
+  };
+  size_t scale[2], flags[2], rest[2];
+  for (int i = 0; i < 2; ++i) {
+    side[i]->rows = i ? rows_b : rows_a;
+    side[i]->rp = (int)vtlb_round_up((size_t)side[i]->rows, 256);
+    const size_t n = blocks * side[i]->rp;
+    scale[i] = piece(n * sizeof(float) / (i ? gemm::kHalfGroup : 1));
+    flags[i] = piece(n / 4);
+    rest[i] = piece(n * gemm::kHalfRest * sizeof(int2));
+  }
+  const size_t extra = piece(extra_bytes);
+  if (int rc = alloc_planes(ctx, rows_a, rows_b, K, behind, &p->tf32)) return rc;
+  char* base = (char*)((uintptr_t)p->tf32.extra & ~(uintptr_t)255);  // pieces start 256 bytes further on
+  for (int i = 0; i < 2; ++i) {
+    // a pair of f16 planes takes no more than the pair of TF32 planes in whose place it lies
+    const size_t n = (size_t)side[i]->rows * p->ld;
+    side[i]->hi = (__half*)(i ? p->tf32.b_hi : p->tf32.a_hi);
+    side[i]->lo = side[i]->hi + vtlb_round_up(n, 128);
+    side[i]->scale = (float*)(base + scale[i]);
+    side[i]->flags = (uint8_t*)(base + flags[i]);
+    side[i]->rest = (int2*)(base + rest[i]);
+  }
+  p->extra = base + extra;
   return VTLB_OK;
 }
 
@@ -190,14 +212,20 @@ int launch_f16x3(vtlb_ctx* ctx, const HalfPlanes& p, int M, int N, int K, Epi ep
   epi.planes = 0;
   if ((rc = prepare_epilogue(ctx, &tm, &epi, M, N, fused))) return rc;
   const uint64_t stride = (uint64_t)p.ld * 2, inner = (uint64_t)K * 2;  // bytes
-  if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[0], false, p.a_hi, inner, M, stride, 128, gemm::BM))) return rc;
-  if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[1], false, p.a_lo, inner, M, stride, 128, gemm::BM))) return rc;
-  if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[0], false, p.b_hi, inner, N, stride, 128, 128))) return rc;
-  if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[1], false, p.b_lo, inner, N, stride, 128, 128))) return rc;
-  const gemm::HalfScales sc{p.a_scale, p.b_scale, p.lda_scale, p.ldb_scale, ctx->d_status + vtlb_ctx::kUnfitWord, epoch};
-  if ((rc = gemm2::launch_pair<gemm::KIND_F16X3, Epi>(ctx, tm, epi, M, N, K, 0, false, sc))) return rc;
+  if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[0], false, p.a.hi, inner, M, stride, 128, gemm::BM))) return rc;
+  if ((rc = gemm::encode_tmap_2d(ctx, &tm.a[1], false, p.a.lo, inner, M, stride, 128, gemm::BM))) return rc;
+  if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[0], false, p.b.hi, inner, N, stride, 128, 128))) return rc;
+  if ((rc = gemm::encode_tmap_2d(ctx, &tm.b[1], false, p.b.lo, inner, N, stride, 128, 128))) return rc;
+  gemm::HalfOperands ho;
+  ho.a = {p.a.hi, p.a.lo, p.a.scale, p.a.flags, p.a.rest, p.a.rp};
+  ho.b = {p.b.hi, p.b.lo, p.b.scale, p.b.flags, p.b.rest, p.b.rp};
+  ho.ld = p.ld;
+  ho.unfit = ctx->d_status + vtlb_ctx::kUnfitWord;
+  ho.listed = ctx->d_status + vtlb_ctx::kListedWord;
+  ho.epoch = epoch;
+  if ((rc = gemm2::launch_pair<gemm::KIND_F16X3, Epi>(ctx, tm, epi, M, N, K, 0, false, ho))) return rc;
   if ((rc = encode_tf32_pair(ctx, &tm, p.tf32, M, N, K))) return rc;
-  return gemm2::launch_pair<gemm::KIND_TF32X3, Epi>(ctx, tm, epi, M, N, K, 0, false, sc);
+  return gemm2::launch_pair<gemm::KIND_TF32X3, Epi>(ctx, tm, epi, M, N, K, 0, false, ho);
 }
 
 // Epilogue: y = acc + bias[col] (one f32 add, as the reference's broadcast add on the

@@ -19,6 +19,7 @@
 // still in flight, frees its tensor memory and returns.
 #pragma once
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -58,15 +59,26 @@ struct Traits<KIND_F16X3> {
 };
 constexpr int kHalfBlock = 256;    // elements of K that share a scale
 constexpr int kHalfGroup = 32;     // rows of B (columns of D) that share one too: a chunk of the epilogue
+constexpr int kHalfRest = 4;       // elements of a row's block that two f16 may leave a rest of
+constexpr int kHalfShift = 12;     // lo planes hold 2^12 times what hi leaves
 
-// What a product on f16 planes needs beside them: the factors that undo the scaling, a[block of K][row of A] and
-// b[block of K][group of rows of B], and the word by which the split passes say that f16 cannot hold the operands
-// (it then equals `epoch`, and the product is left to the 3xTF32 kernel launched behind it).
-struct HalfScales {
-  const float* a = nullptr;
-  const float* b = nullptr;
-  int lda = 0, ldb = 0;
-  const uint32_t* unfit = nullptr;
+// One operand on f16 planes, K-major; `rp` is its number of rows rounded up to whole tiles of 256.
+struct HalfSide {
+  const __half *hi, *lo;   // [rows][ld]
+  const float* scale;      // what undoes the scaling: A [block of K][rp], B [block of K][rp / kHalfGroup]
+  // Elements that the planes do not hold to 22 bits: bit q of flags[block][row / 4] says that row 4 * (row / 4) + q has
+  // some, rest[block][row][kHalfRest] are {k, x - what is held}, k = -1 behind the last
+  const uint8_t* flags;    // [block of K][rp / 4]
+  const int2* rest;        // [block of K][rp][kHalfRest]
+  int rp;
+};
+// What a product on f16 planes needs beside the tensor maps, and two words that the split passes set to `epoch`: *unfit
+// when f16 cannot hold the operands (the product is then left to the 3xTF32 kernel launched behind it), *listed when
+// there are rests.
+struct HalfOperands {
+  HalfSide a = {}, b = {};
+  int ld = 0;
+  const uint32_t *unfit = nullptr, *listed = nullptr;
   uint32_t epoch = 0;
 };
 

@@ -13,7 +13,8 @@
 // (only in the leader CTA) and tensor-memory owner, warps 2..9 epilogue.  Cross-CTA
 // signalling:
 //   full[s]    lives in the leader; both CTAs' TMA loads complete their bytes on it
-//   empty[s]   one per CTA; the leader's tcgen05.commit multicasts the arrive to both
+//   empty[s]   one per CTA; the leader's tcgen05.commit multicasts the arrive to both (f16 planes: lo[s] too,
+//              for the lo planes alone)
 //   tfull[a]   one per CTA; commit multicast
 //   tempty[a]  lives in the leader; the 16 epilogue warps of the pair arrive on it
 // No TMA multicast is used: every CTA issues plain loads into its own shared memory.
@@ -46,7 +47,9 @@ struct Cfg {
   static constexpr uint32_t STAGE = NOP * (A_TILE + B_HALF);          // 32 KB (INT8) / 64 KB (TF32x3)
   static constexpr uint32_t TILES = STAGES * STAGE;
   static constexpr uint32_t BARS_OFF = TILES + gemm::STAGING;         // epilogue staging tiles in between
-  static constexpr uint32_t SMEM_TOTAL = BARS_OFF + 8 * (2 * STAGES + 4) + 16 + 1024;
+  // full, empty, two each of tfull and tempty, and for f16 planes: lo planes empty
+  static constexpr int NUM_BARS = 2 * STAGES + 4 + (KIND == gemm::KIND_F16X3 ? STAGES : 0);
+  static constexpr uint32_t SMEM_TOTAL = BARS_OFF + 8 * NUM_BARS + 16 + 1024;
   // TF32x3 closes its accumulator every CHUNK_KB stages (the f32 accumulate of tcgen05 truncates;
   // see gemm_tc.cuh).  With 256 columns per accumulator and two buffers there is no room in tensor
   // memory for a separate accumulator of the small cross terms: here they share the main one, which
@@ -135,6 +138,17 @@ __device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t adesc, u
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// D = D / 2^kHalfShift + A.B
+__device__ __forceinline__ void umma_f16_pair_shift(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.eq.b32 p, 0, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, %4;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "n"(gemm::kHalfShift)
+      : "memory");
+}
 __device__ __forceinline__ void umma_i8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                              uint32_t accumulate) {
   asm volatile(
@@ -181,12 +195,112 @@ __device__ __forceinline__ bool flag_wait_bounded(const uint32_t* flag, uint32_t
   }
 }
 
+// Bits of the rows (0 .. 31, bit 8 * (row / 4) + row % 4) of a group of 32 that have elements listed in a block.
+__device__ __forceinline__ uint64_t rest_flags(const gemm::HalfSide& s, int blk, int row) {
+  return __ldg(reinterpret_cast<const unsigned long long*>(s.flags + ((size_t)blk * s.rp + row) / 4)) &
+         0x0f0f0f0f0f0f0f0full;
+}
+__device__ __forceinline__ float half_kept(const gemm::HalfSide& s, int ld, int row, int k, float scale) {
+  const size_t at = (size_t)row * ld + k;
+  return __fmaf_rn(__half2float(__ldg(s.lo + at)), 1.0f / (1 << gemm::kHalfShift), __half2float(__ldg(s.hi + at))) * scale;
+}
+// The products of the elements that the f16 planes do not hold (gemm::HalfSide::rest): to this warp's 32 rows x four
+// chunks of 32 columns (64 apart, the first at col0), rest(a) * b with all of b, and what is held of a * rest(b).  The
+// sums start with them, so the loads run beside the tile's first MMAs.  Each costs a round of loads and an addition,
+// predicated, per value.  A fixed order, so results repeat.
+__device__ __forceinline__ void add_rests(float (&sum)[BN2 / 2], const gemm::HalfOperands& o, int row0, int col0,
+                                          int lane, int M, int N, int K) {
+  constexpr int NC = BN2 / 64, G = gemm::kHalfGroup;
+  const int blocks = (K + gemm::kHalfBlock - 1) / gemm::kHalfBlock;
+  const int my_bit = lane / 4 * 8 + lane % 4;
+  for (int b0 = 0; b0 < blocks; b0 += 32) {  // a lane looks one block over
+    const int mine = b0 + lane < blocks ? b0 + lane : b0;
+    uint64_t any = rest_flags(o.a, mine, row0);
+#pragma unroll
+    for (int cc = 0; cc < NC; ++cc) any |= rest_flags(o.b, mine, col0 + cc * 64);
+    uint32_t todo = __ballot_sync(0xffffffffu, b0 + lane < blocks && any != 0);
+    while (todo) {
+      const int blk = b0 + __ffs(todo) - 1;
+      todo &= todo - 1;
+      // what lies behind the last row or column was never written
+      const int row = row0 + lane;
+      const uint32_t rows = __ballot_sync(0xffffffffu, row < M && (rest_flags(o.a, blk, row0) >> my_bit & 1));
+      if (rows) {
+        const int2* list = o.a.rest + ((size_t)blk * o.a.rp + row) * gemm::kHalfRest;
+#pragma unroll 1
+        for (int e = 0; e < gemm::kHalfRest; ++e) {  // a lane its own row's
+          const int2 it = rows >> lane & 1u ? __ldg(list + e) : make_int2(-1, 0);
+          uint32_t have = __ballot_sync(0xffffffffu, it.x >= 0);
+          if (!have) break;
+#pragma unroll 1
+          for (; have; have &= have - 1) {
+            const int r = __ffs(have) - 1, k = __shfl_sync(0xffffffffu, it.x, r);
+            const float rest = __int_as_float(__shfl_sync(0xffffffffu, it.y, r));
+            float b[NC];
+            bool more = false;
+#pragma unroll
+            for (int cc = 0; cc < NC; ++cc) {  // the loads of all four chunks together
+              const int n = col0 + cc * 64 + lane, at = n < N ? n : N - 1;
+              b[cc] = half_kept(o.b, o.ld, at, k, __ldg(o.b.scale + ((size_t)blk * o.b.rp + at) / G));
+              more = more || (n < N && (rest_flags(o.b, blk, col0 + cc * 64) >> my_bit & 1));
+            }
+            if (__any_sync(0xffffffffu, more)) {  // the column may have a rest at the same k
+#pragma unroll
+              for (int cc = 0; cc < NC; ++cc) {
+                const int n = col0 + cc * 64 + lane;
+                if (n >= N || !(rest_flags(o.b, blk, col0 + cc * 64) >> my_bit & 1)) continue;
+                const int2* lb = o.b.rest + ((size_t)blk * o.b.rp + n) * gemm::kHalfRest;
+                for (int i = 0; i < gemm::kHalfRest; ++i) {
+                  const int2 jt = __ldg(lb + i);
+                  if (jt.x < 0) break;
+                  if (jt.x == k) b[cc] += __int_as_float(jt.y);
+                }
+              }
+            }
+#pragma unroll
+            for (int cc = 0; cc < NC; ++cc) {
+              const float p = b[cc] * rest;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const float t = __shfl_sync(0xffffffffu, p, j);
+                if (lane == r) sum[cc * 32 + j] += t;
+              }
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int cc = 0; cc < NC; ++cc) {
+        const int n = col0 + cc * 64 + lane;
+        const uint32_t cols =
+            __ballot_sync(0xffffffffu, n < N && (rest_flags(o.b, blk, col0 + cc * 64) >> my_bit & 1));
+        if (!cols) continue;
+        const int2* list = o.b.rest + ((size_t)blk * o.b.rp + n) * gemm::kHalfRest;
+#pragma unroll 1
+        for (int e = 0; e < gemm::kHalfRest; ++e) {  // a lane its own column's
+          const int2 it = cols >> lane & 1u ? __ldg(list + e) : make_int2(-1, 0);
+          uint32_t have = __ballot_sync(0xffffffffu, it.x >= 0);
+          if (!have) break;
+#pragma unroll 1
+          for (; have; have &= have - 1) {
+            const int c = __ffs(have) - 1, k = __shfl_sync(0xffffffffu, it.x, c);
+            float p = __int_as_float(__shfl_sync(0xffffffffu, it.y, c));
+            p *= row < M ? half_kept(o.a, o.ld, row, k, __ldg(o.a.scale + (size_t)blk * o.a.rp + row)) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (c == j) sum[cc * 32 + j] += p;
+          }
+        }
+      }
+    }
+  }
+}
 
 template <int KIND, class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M, int N, int K,
                  int group_m, int a_chunk_k, int split_tiles, uint32_t* ksplit_buf, uint32_t ksplit_epoch,
-                 uint32_t* status, const gemm::HalfScales sc) {
+                 uint32_t* status, const gemm::HalfOperands ho) {
   using T = gemm::Traits<KIND>;
   using C = Cfg<KIND>;
   constexpr int NOP = C::NOP, STAGES = C::STAGES;
@@ -197,7 +311,7 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
 
   // one of the two kernels launched for a product on f16 planes leaves at once; both CTAs of a pair read the same
   // (those launches do not start early, so the word may be read before the wait below)
-  if (KIND != gemm::KIND_I8 && sc.unfit != nullptr && (*sc.unfit == sc.epoch) != (KIND == gemm::KIND_TF32X3)) return;
+  if (KIND != gemm::KIND_I8 && ho.unfit != nullptr && (*ho.unfit == ho.epoch) != (KIND == gemm::KIND_TF32X3)) return;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -207,7 +321,8 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
   auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
   auto tfull_bar = [&](int a) { return bars + 8u * (2 * STAGES + a); };
   auto tempty_bar = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (bars - raw) + 8u * (2 * STAGES + 4));
+  auto lo_empty_bar = [&](int s) { return bars + 8u * (2 * STAGES + 4 + s); };  // f16 planes only
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (bars - raw) + 8u * C::NUM_BARS);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -268,6 +383,7 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
     for (int s = 0; s < STAGES; ++s) {
       ptx::mbar_init(full_bar(s), 1);   // the leader's expect_tx arrive; bytes from both CTAs
       ptx::mbar_init(empty_bar(s), 1);  // one multicast commit
+      if (KIND == gemm::KIND_F16X3) ptx::mbar_init(lo_empty_bar(s), 1);
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(tfull_bar(a), 1);
@@ -306,7 +422,8 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
         const int m0 = tmi * 2 * BM + (int)rank * BM;
         const int n0 = tni * BN2 + (int)rank * (BN2 / 2);
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!ptx::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag, WAIT_LIMIT_NS)) {
+          if (!ptx::mbar_wait_bounded(KIND == gemm::KIND_F16X3 ? lo_empty_bar(stage) : empty_bar(stage), phase ^ 1u,
+                                      abort_flag, WAIT_LIMIT_NS)) {
             ok = false;
             break;
           }
@@ -314,17 +431,29 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
           if (rank == 0) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * C::STAGE);
           const uint32_t sa = base + stage * C::STAGE;
           const uint32_t sb = sa + NOP * C::A_TILE;
+          if constexpr (KIND == gemm::KIND_F16X3) {
+            // the lo planes of a stage are free two thirds of a chunk before its hi planes (see the MMA warp)
+            tma_load_2d_pair(sa + C::A_TILE, &tm.a[1], kb * XSTEP, m0, leader_full);
+            tma_load_2d_pair(sb + C::B_HALF, &tm.b[1], kb * XSTEP, n0, leader_full);
+            if (!ptx::mbar_wait_bounded(empty_bar(stage), phase ^ 1u, abort_flag, WAIT_LIMIT_NS)) {
+              ok = false;
+              break;
+            }
+            tma_load_2d_pair(sa, &tm.a[0], kb * XSTEP, m0, leader_full);
+            tma_load_2d_pair(sb, &tm.b[0], kb * XSTEP, n0, leader_full);
+          } else {
 #pragma unroll
-          for (int i = 0; i < NOP; ++i) {
-            if (a_chunk_k)  // A stored as [chunk][M][a_chunk_k] (gathered column shards)
-              tma_load_3d_pair(sa + i * C::A_TILE, &tm.a[i], (kb * BK) % a_chunk_k, m0, (kb * BK) / a_chunk_k,
-                               leader_full);
-            else
-              tma_load_2d_pair(sa + i * C::A_TILE, &tm.a[i], kb * XSTEP, m0, leader_full);
+            for (int i = 0; i < NOP; ++i) {
+              if (a_chunk_k)  // A stored as [chunk][M][a_chunk_k] (gathered column shards)
+                tma_load_3d_pair(sa + i * C::A_TILE, &tm.a[i], (kb * BK) % a_chunk_k, m0, (kb * BK) / a_chunk_k,
+                                 leader_full);
+              else
+                tma_load_2d_pair(sa + i * C::A_TILE, &tm.a[i], kb * XSTEP, m0, leader_full);
+            }
+#pragma unroll
+            for (int i = 0; i < NOP; ++i)
+              tma_load_2d_pair(sb + i * C::B_HALF, &tm.b[i], kb * XSTEP, n0, leader_full);
           }
-#pragma unroll
-          for (int i = 0; i < NOP; ++i)
-            tma_load_2d_pair(sb + i * C::B_HALF, &tm.b[i], kb * XSTEP, n0, leader_full);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
@@ -349,6 +478,10 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
           }
           ptx::tc_fence_after();
           const uint32_t d_tmem = tmem_base + acc * BN2;
+          // f16 planes: first the cross terms of the whole chunk, which are 2^12 times too large, then hi.hi, whose
+          // first MMA takes the factor back.  A stage's lo planes are free after its cross terms, its hi planes after
+          // hi.hi: with three stages, chunks of two and one barrier for both the loads came 1.5 to 2 % late.
+          const uint32_t first_stage = stage;
           for (int kb = kb0; kb < kb1; ++kb) {
             if (!ptx::mbar_wait_bounded(full_bar(stage), phase, abort_flag, WAIT_LIMIT_NS)) {
               ok = false;
@@ -370,20 +503,35 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
                 const uint64_t b_hi = ptx::umma_desc_k_sw128(sb) + 2u * kk;
                 const uint64_t b_lo = ptx::umma_desc_k_sw128(sb + C::B_HALF) + 2u * kk;
                 if constexpr (KIND == gemm::KIND_F16X3) {
-                  umma_f16_pair(d_tmem, a_lo, b_hi, IDESC, first);  // small terms first
+                  umma_f16_pair(d_tmem, a_lo, b_hi, IDESC, first);
                   umma_f16_pair(d_tmem, a_hi, b_lo, IDESC, 1);
-                  umma_f16_pair(d_tmem, a_hi, b_hi, IDESC, 1);
                 } else {
-                  umma_tf32_pair(d_tmem, a_lo, b_hi, IDESC, first);
+                  umma_tf32_pair(d_tmem, a_lo, b_hi, IDESC, first);  // small terms first
                   umma_tf32_pair(d_tmem, a_hi, b_lo, IDESC, 1);
                   umma_tf32_pair(d_tmem, a_hi, b_hi, IDESC, 1);
                 }
               }
             }
-            umma_commit_pair(empty_bar(stage));
+            umma_commit_pair(KIND == gemm::KIND_F16X3 ? lo_empty_bar(stage) : empty_bar(stage));
             if (++stage == STAGES) {
               stage = 0;
               phase ^= 1u;
+            }
+          }
+          if constexpr (KIND == gemm::KIND_F16X3) {
+            uint32_t st = first_stage;
+            for (int kb = kb0; kb < kb1 && ok; ++kb) {
+              const uint32_t sa = base + st * C::STAGE;
+              const uint32_t sb = sa + NOP * C::A_TILE;
+#pragma unroll
+              for (int kk = 0; kk < KSTEPS; ++kk) {
+                const uint64_t a_hi = ptx::umma_desc_k_sw128(sa) + 2u * kk;
+                const uint64_t b_hi = ptx::umma_desc_k_sw128(sb) + 2u * kk;
+                if (kb == kb0 && kk == 0) umma_f16_pair_shift(d_tmem, a_hi, b_hi, IDESC);
+                else umma_f16_pair(d_tmem, a_hi, b_hi, IDESC, 1);
+              }
+              umma_commit_pair(empty_bar(st));
+              if (++st == STAGES) st = 0;
             }
           }
           if (!ok) break;
@@ -401,6 +549,7 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
     const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
     uint32_t acc = 0, acc_phase = 0;
     bool ok = true;
+    const bool listed = KIND == gemm::KIND_F16X3 && *ho.listed == ho.epoch;
     for (int it = 0; ok; ++it) {
       int tmi, tni, kh, slot;
       if (!decode_unit(it, tmi, tni, kh, slot)) break;
@@ -469,6 +618,8 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
         float sum[BN2 / 2];  // this warp's four 32-column chunks
 #pragma unroll
         for (int j = 0; j < BN2 / 2; ++j) sum[j] = 0.0f;
+        if constexpr (KIND == gemm::KIND_F16X3)
+          if (listed) add_rests(sum, ho, row0, n0 + half * 32, lane, M, N, K);
         // ReLU-backward mask of the tile's outputs, fetched now as one bit per value
         uint32_t mask_bits[BN2 / 64];
         if constexpr (gemm::EpiHasPlanes<Epi>::value) {
@@ -485,10 +636,10 @@ gemm_pair_kernel(const __grid_constant__ gemm::TmapSet tm, const Epi epi, int M,
           float f[BN2 / 64];
           if constexpr (KIND == gemm::KIND_F16X3) {
             const int blk = kb0 / C::SCALE_KB;
-            const float fa = __ldg(sc.a + (size_t)blk * sc.lda + row0 + lane);
+            const float fa = __ldg(ho.a.scale + (size_t)blk * ho.a.rp + row0 + lane);
 #pragma unroll
             for (int cc = 0; cc < BN2 / 64; ++cc)
-              f[cc] = __fmul_rn(fa, __ldg(sc.b + (size_t)blk * sc.ldb + n0 / gemm::kHalfGroup + 2 * cc + half));
+              f[cc] = __fmul_rn(fa, __ldg(ho.b.scale + ((size_t)blk * ho.b.rp + n0) / gemm::kHalfGroup + 2 * cc + half));
           }
           ok = ptx::mbar_wait_bounded(tfull_bar(acc), acc_phase, abort_flag, WAIT_LIMIT_NS);
           ok = __all_sync(0xffffffffu, ok);
@@ -562,7 +713,7 @@ inline bool pair_worthwhile(vtlb_ctx* ctx, int M, int N) {
 
 template <int KIND, class Epi>
 int launch_pair(vtlb_ctx* ctx, const gemm::TmapSet& tm, const Epi& epi, int M, int N, int K,
-                int a_chunk_k = 0, bool k_split = false, const gemm::HalfScales& sc = gemm::HalfScales()) {
+                int a_chunk_k = 0, bool k_split = false, const gemm::HalfOperands& ho = gemm::HalfOperands()) {
   using C = Cfg<KIND>;
   static_assert(C::SMEM_TOTAL <= 232448, "shared memory budget");
   auto kern = gemm_pair_kernel<KIND, Epi>;
@@ -576,7 +727,7 @@ int launch_pair(vtlb_ctx* ctx, const gemm::TmapSet& tm, const Epi& epi, int M, i
   if (tiles < pairs) pairs = tiles;
   // (a 3xTF32 launch behind a product on f16 planes is that product once more, if at all)
   const bool timed = ctx->prof_on && ctx->prof_ev && ctx->prof_n < vtlb_ctx::kProfSlots &&
-                     !(KIND == gemm::KIND_TF32X3 && sc.unfit);
+                     !(KIND == gemm::KIND_TF32X3 && ho.unfit);
   if (timed) cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n], ctx->stream);
   const int group_m = gemm::pick_group_m((M + 2 * BM - 1) / (2 * BM),
                                          (size_t)2 * BM * K * gemm::Traits<KIND>::ELEM * C::NOP);
@@ -594,11 +745,11 @@ int launch_pair(vtlb_ctx* ctx, const gemm::TmapSet& tm, const Epi& epi, int M, i
   if (tiles <= pairs && KIND == gemm::KIND_I8)
     VTLB_CUDA(ctx, vtlb_launch_early(kern, dim3(2 * pairs), dim3(NUM_THREADS), C::SMEM_TOTAL, ctx->stream, tm, epi, M, N, K,
                                      group_m, a_chunk_k, split_tiles, (uint32_t*)ctx->ksplit_buf, ctx->ksplit_epoch,
-                                     ctx->d_status, sc));
+                                     ctx->d_status, ho));
   else
     kern<<<2 * pairs, NUM_THREADS, C::SMEM_TOTAL, ctx->stream>>>(tm, epi, M, N, K, group_m, a_chunk_k, split_tiles,
                                                                  (uint32_t*)ctx->ksplit_buf, ctx->ksplit_epoch,
-                                                                 ctx->d_status, sc);
+                                                                 ctx->d_status, ho);
   if (timed) {
     cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n + 1], ctx->stream);
     ctx->prof_n++;
