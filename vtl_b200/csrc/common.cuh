@@ -201,4 +201,9 @@ __device__ __forceinline__ bool vtlb_last_block(uint32_t* ticket) {
 #endif
 
 static inline bool vtlb_aligned16(const void* p) { return (((uintptr_t)p) & 15u) == 0; }
+// Two arrays of f32 that share memory.
+static inline bool vtlb_overlap(const void* a, size_t na, const void* b, size_t nb) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + nb * sizeof(float) && y < x + na * sizeof(float);
+}
 static inline size_t vtlb_round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }

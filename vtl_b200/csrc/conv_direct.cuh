@@ -373,10 +373,12 @@ int launch_wgrad_t(vtlb_ctx* ctx, const float* g, const float* x, float* dW, int
   const size_t n = (size_t)O * C * K * K;
   void* scr = nullptr;
   if (int rc = vtlb_scratch(ctx, (size_t)parts * n * sizeof(float), &scr)) return rc;
+  // a dW over x or g is written when both have been read, as by the kernels that this one stands in for
+  const bool by_scratch = parts > 1 || vtlb_overlap(dW, n, x, (size_t)B * C * H * W) || vtlb_overlap(dW, n, g, (size_t)B * O * Ho * Wo);
   VTLB_CUDA(ctx, vtlb_launch_early(wgrad_direct_kernel<K, OT>, dim3(parts, C, og), dim3(kThreads), 0, ctx->stream, g, x, C,
-                                   H, W, O, Ho, Wo, ph, pw, sh, sw, pixels, per, parts > 1 ? (float*)scr : dW));
+                                   H, W, O, Ho, Wo, ph, pw, sh, sw, pixels, per, by_scratch ? (float*)scr : dW));
   VTLB_LAUNCHED(ctx);
-  return parts > 1 ? f32::reduce_splits(ctx, (const float*)scr, parts, n, dW) : VTLB_OK;
+  return by_scratch ? f32::reduce_splits(ctx, (const float*)scr, parts, n, dW) : VTLB_OK;
 }
 inline int launch_wgrad(vtlb_ctx* ctx, const float* g, const float* x, float* dW, int B, int C, int H, int W, int O,
                         int Ho, int Wo, int K, int ph, int pw, int sh, int sw) {

@@ -536,7 +536,15 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
   const int ld_rows = vtlb_plane_ld(N), ld_cols = vtlb_plane_ld(M);
   int rc, fused = 0;
   const bool planes_in_or_out = ex.a_planes || ex.b_planes || ex.out_rows || ex.out_cols;
-  const bool small = small_product(ctx, M, N, K);
+  bool small = small_product(ctx, M, N, K);
+  if (small && 2.0 * M * N * K > ctx->small_gemm_flops) {
+    // CUDA cores read the operands while C is written.  Above the limit a result may lie over an operand: the
+    // tensor-core routes have copied both before they write.
+    auto over = [&](const float* out) {
+      return vtlb_overlap(out, (size_t)M * N, A, (size_t)M * K) || vtlb_overlap(out, (size_t)M * N, B, (size_t)N * K);
+    };
+    small = !over(C) && !(pre && over(pre));
+  }
   if (!small && !planes_in_or_out && gemm2::pair_worthwhile(ctx, M, N)) {
     // Large products: f16 planes on CTA pairs, twice the tensor rate of TF32 planes and half their bytes.  Planes
     // that come in or go out are TF32 ones, so products with those keep the 3xTF32 kernel.
@@ -549,11 +557,6 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
     const uint32_t epoch = ctx->half_epoch;
     if ((rc = split_operand_half(ctx, A, K, transA != 0, false, p.ld, p.a, partial, epoch))) return rc;
     if ((rc = split_operand_half(ctx, B, K, transB == 0, true, p.ld, p.b, nullptr, epoch))) return rc;
-    if (sums) {
-      colsum_final_kernel<<<(M + 127) / 128, 128, 0, ctx->stream>>>(partial, blocks, M, ex.a_colsum);
-      VTLB_LAUNCHED(ctx);
-      *ex.colsum_done = true;
-    }
     {
       const SplitSource sa{A, p.tf32.a_hi, p.tf32.a_lo, M, K, p.tf32.ld, transA != 0};
       const SplitSource sb{B, p.tf32.b_hi, p.tf32.b_lo, N, K, p.tf32.ld, transB == 0};
@@ -564,6 +567,11 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
     f32::EpiBiasRelu epi{C, bias, pre, N, relu};
     epi.mask = ex.mask;
     if ((rc = f32::launch_f16x3(ctx, p, M, N, K, epi, epoch, &fused))) return rc;
+    if (sums) {  // written last, as by a pass of its own
+      colsum_final_kernel<<<(M + 127) / 128, 128, 0, ctx->stream>>>(partial, blocks, M, ex.a_colsum);
+      VTLB_LAUNCHED(ctx);
+      *ex.colsum_done = true;
+    }
   } else if (small) {  // launch-latency-bound sizes: CUDA cores, no split passes
     if ((rc = f32::sgemm_small(ctx, transA, transB, M, N, K, A, B, C, bias, relu, pre, nullptr, nullptr, ex.mask)))
       return rc;
@@ -690,11 +698,6 @@ int linear_fwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_X, const void* 
                        (const float*)d_b_or_null, relu, (float*)d_pre_or_null, ex);
 }
 
-bool overlap(const void* a, size_t na, const void* b, size_t nb) {  // arrays of f32
-  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
-  return x < y + nb * sizeof(float) && y < x + na * sizeof(float);
-}
-
 int linear_bwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_G, const void* d_X, const void* d_W,
                     void* d_dX_or_null, void* d_dW_or_null, void* d_db_or_null, int M, int N, int K,
                     const vtlb_planes* g_rows, const vtlb_planes* g_cols, const vtlb_planes* x_cols,
@@ -726,13 +729,24 @@ int linear_bwd_impl(vtlb_ctx* ctx, const char* fn, const void* d_G, const void* 
     d_db_or_null = nullptr;
   }
   bool db_done = false;
-  // a small layer: both products in one launch, where neither writes what the other reads
-  if (!any_planes && small_backward(ctx, M, N, K) && d_dX_or_null && d_dW_or_null && d_W && d_X && vtlb_aligned16(d_dX_or_null) && vtlb_aligned16(d_dW_or_null) &&
-      !overlap(d_dX_or_null, (size_t)M * K, d_X, (size_t)M * K) && !overlap(d_dX_or_null, (size_t)M * K, d_G, (size_t)M * N) &&
-      !overlap(d_dW_or_null, (size_t)N * K, d_W, (size_t)N * K) && !overlap(d_dW_or_null, (size_t)N * K, d_G, (size_t)M * N) &&
-      !(d_relu_mask_src_or_null && overlap(d_dW_or_null, (size_t)N * K, d_relu_mask_src_or_null, (size_t)M * K)) &&
-      !(d_db_or_null && (overlap(d_db_or_null, (size_t)N, d_W, (size_t)N * K) ||
-                         overlap(d_db_or_null, (size_t)N, d_G, (size_t)M * N)))) {
+  // a small layer: both products in one launch, where no result lies over another or over what is read (the mask may be
+  // dX itself: each value is read by the thread that writes it)
+  const void *outs[3] = {d_dX_or_null, d_dW_or_null, d_db_or_null};
+  const size_t out_n[3] = {(size_t)M * K, (size_t)N * K, (size_t)N};
+  auto apart = [&] {
+    const void* ins[4] = {d_G, d_X, d_W, d_relu_mask_src_or_null};
+    const size_t in_n[4] = {(size_t)M * N, (size_t)M * K, (size_t)N * K, (size_t)M * K};
+    for (int o = 0; o < 3; ++o) {
+      for (int i = 0; i < 4; ++i)
+        if (outs[o] && ins[i] && !(o == 0 && i == 3 && outs[o] == ins[i]) && vtlb_overlap(outs[o], out_n[o], ins[i], in_n[i]))
+          return false;
+      for (int p = 0; p < o; ++p)
+        if (outs[o] && outs[p] && vtlb_overlap(outs[o], out_n[o], outs[p], out_n[p])) return false;
+    }
+    return true;
+  };
+  if (!any_planes && small_backward(ctx, M, N, K) && d_dX_or_null && d_dW_or_null && d_W && d_X &&
+      vtlb_aligned16(d_dX_or_null) && vtlb_aligned16(d_dW_or_null) && apart()) {
     bool done = false;
     if ((rc = f32::sgemm_small_linear_bwd(ctx, (const float*)d_G, (const float*)d_X, (const float*)d_W,
                                           (float*)d_dX_or_null, (float*)d_dW_or_null, (float*)d_db_or_null, M, N, K,
