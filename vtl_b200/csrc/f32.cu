@@ -16,11 +16,8 @@ namespace {
 using f32::split1;
 
 // src [R, C] row-major (C % 4 == 0, 16-byte aligned) -> hi/lo [R, C].  12 bytes/element.
-__global__ void __launch_bounds__(256) split_rows_vec_kernel(const float4* __restrict__ src,
-                                                             float4* __restrict__ hi,
-                                                             float4* __restrict__ lo, size_t n4) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__device__ __forceinline__ void split_rows_vec(const float4* __restrict__ src, float4* __restrict__ hi,
+                                               float4* __restrict__ lo, size_t n4) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4;
        i += (size_t)gridDim.x * blockDim.x) {
     float4 x = src[i], h, l;
@@ -32,13 +29,9 @@ __global__ void __launch_bounds__(256) split_rows_vec_kernel(const float4* __res
     lo[i] = l;
   }
 }
-
 // General case: src [R, C] -> hi/lo [R, ldo], ldo >= C.
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ src, int R,
-                                                         int C, int ldo, float* __restrict__ hi,
-                                                         float* __restrict__ lo) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__device__ __forceinline__ void split_rows(const float* __restrict__ src, int R, int C, int ldo, float* __restrict__ hi,
+                                           float* __restrict__ lo) {
   const size_t n = (size_t)R * C;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
@@ -49,16 +42,10 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
     lo[r * ldo + c] = l;
   }
 }
-
 // src [R, C] row-major -> hi/lo [C, ldo] (the transpose), ldo >= R.  32x32 tiles
 // through shared memory so that both the reads and the writes are coalesced.
-__global__ void __launch_bounds__(256) split_transpose_kernel(const float* __restrict__ src, int R,
-                                                              int C, int ldo,
-                                                              float* __restrict__ hi,
-                                                              float* __restrict__ lo) {
-  __shared__ float tile[32][33];
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+__device__ __forceinline__ void split_transpose(const float* __restrict__ src, int R, int C, int ldo,
+                                                float* __restrict__ hi, float* __restrict__ lo, float (&tile)[32][33]) {
   const int tiles_c = (C + 31) / 32, tiles_r = (R + 31) / 32;
   const long long ntiles = (long long)tiles_c * tiles_r;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -82,6 +69,26 @@ __global__ void __launch_bounds__(256) split_transpose_kernel(const float* __res
     }
     __syncthreads();
   }
+}
+
+__global__ void __launch_bounds__(256) split_rows_vec_kernel(const float4* __restrict__ src, float4* __restrict__ hi,
+                                                             float4* __restrict__ lo, size_t n4) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  split_rows_vec(src, hi, lo, n4);
+}
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ src, int R, int C, int ldo,
+                                                         float* __restrict__ hi, float* __restrict__ lo) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  split_rows(src, R, C, ldo, hi, lo);
+}
+__global__ void __launch_bounds__(256) split_transpose_kernel(const float* __restrict__ src, int R, int C, int ldo,
+                                                              float* __restrict__ hi, float* __restrict__ lo) {
+  __shared__ float tile[32][33];
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early (vtlb_launch_early): the kernel in front is done
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  split_transpose(src, R, C, ldo, hi, lo, tile);
 }
 
 // The multiplier 2^e that brings a block's largest magnitude into [2^14, 2^15), and 2^-e.  e is kept where both
@@ -119,6 +126,10 @@ struct HalfOut {
   uint32_t *count, *unfit, *listed;
   uint32_t limit, epoch;
 };
+// True in every thread once the product is known to be unfit: nothing is left to do then.
+__device__ __forceinline__ bool known_unfit(const HalfOut& o) {
+  return __syncthreads_or(threadIdx.x == 0 && *(volatile const uint32_t*)o.unfit == o.epoch);
+}
 // One scale of a block: so extreme that the product of two such would leave the f32 range (an infinity in the block
 // among them)?
 __device__ __forceinline__ void note_scale(float mul, const HalfOut& o) {
@@ -196,6 +207,7 @@ __global__ void __launch_bounds__(256) split_rows_half_kernel(const float* __res
         for (int j = 0; j < 8; ++j) v[q][j] = row && c + j < C ? __ldg(a + j) : 0.0f;
       }
     }
+    if (known_unfit(o)) return;  // asked behind the loads, which take as long
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       m[q] = 0.0f;
@@ -266,8 +278,8 @@ __global__ void __launch_bounds__(256) split_transpose_half_kernel(const float* 
       tile[warp + j][lane] = x;
       if (GROUP) all = fmaxf(all, fabsf(x));
     }
+    if (known_unfit(o) && !colsum) return;  // also waits for the tile; the column sums are wanted all the same
     if (GROUP) all = block_amax(all, part);
-    else __syncthreads();
     uint32_t bad = 0;  // bit 8 q + j: element j of column q is not held
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -337,29 +349,14 @@ __global__ void __launch_bounds__(256) split_unfit_kernel(SplitSource a, SplitSo
   __shared__ float tile[32][33];
   if (blockIdx.x == 0 && threadIdx.x < 2) counts[threadIdx.x] = 0;  // listed elements: the next product counts again
   if (*unfit != epoch) return;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int o = 0; o < 2; ++o) {
-    const SplitSource s = o ? b : a;
-    const int tiles_k = (s.kdim + 31) / 32;
-    const long long ntiles = (long long)((s.rows + 31) / 32) * tiles_k;
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      const int r0 = (int)(t / tiles_k) * 32, k0 = (int)(t % tiles_k) * 32;
-      if (s.transposed) {
-        __syncthreads();
-        for (int j = ty; j < 32; j += 8)
-          tile[j][tx] = k0 + j < s.kdim && r0 + tx < s.rows ? s.src[(size_t)(k0 + j) * s.rows + r0 + tx] : 0.0f;
-        __syncthreads();
-      }
-      for (int j = ty; j < 32; j += 8) {
-        const int r = r0 + j, k = k0 + tx;
-        if (r < s.rows && k < s.kdim) {
-          float h, l;
-          split1(s.transposed ? tile[tx][j] : s.src[(size_t)r * s.kdim + k], h, l);
-          s.hi[(size_t)r * s.ld + k] = h;
-          s.lo[(size_t)r * s.ld + k] = l;
-        }
-      }
-    }
+    const SplitSource& s = o ? b : a;
+    if (s.transposed)
+      split_transpose(s.src, s.kdim, s.rows, s.ld, s.hi, s.lo, tile);
+    else if (s.ld == s.kdim && ((uintptr_t)s.src & 15) == 0)
+      split_rows_vec((const float4*)s.src, (float4*)s.hi, (float4*)s.lo, (size_t)s.rows * s.kdim / 4);
+    else
+      split_rows(s.src, s.rows, s.kdim, s.ld, s.hi, s.lo);
   }
 }
 
@@ -560,7 +557,7 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
     {
       const SplitSource sa{A, p.tf32.a_hi, p.tf32.a_lo, M, K, p.tf32.ld, transA != 0};
       const SplitSource sb{B, p.tf32.b_hi, p.tf32.b_lo, N, K, p.tf32.ld, transB == 0};
-      split_unfit_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(sa, sb, ctx->d_status + vtlb_ctx::kUnfitWord, epoch,
+      split_unfit_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(sa, sb, ctx->d_status + vtlb_ctx::kUnfitWord, epoch,
                                                                      ctx->d_status + vtlb_ctx::kRestWord);
       VTLB_LAUNCHED(ctx);
     }
