@@ -186,3 +186,22 @@ def test_scratch_of_a_large_product():
     for b in bufs:
         b.free()
     dev.close()
+
+
+def test_time_of_a_product_that_f16_planes_cannot_hold(dev):
+    """The profile brackets the launches of a product, whichever of them does the work."""
+    M, N, K = 4096, 4096, 4096
+    rng = np.random.default_rng(8)
+    A = (rng.standard_normal((M, K)) * 10.0 ** rng.uniform(-9, 0, (M, K))).astype(np.float32)
+    B = rng.standard_normal((N, K)).astype(np.float32)
+    bufs = [dev.to_device(A), dev.to_device(B), dev.zeros((M, N))]
+    dev.gemm_f32(False, True, M, N, K, *bufs)
+    dev.sync()
+    dev.profile_gemm(True)
+    dev.gemm_f32(False, True, M, N, K, *bufs)
+    ms, launches, ops = dev.profile_gemm_read()
+    dev.profile_gemm(False)
+    assert launches == 1 and ops == 2.0 * M * N * K
+    assert ops / (ms * 1e-3) < 1.0e15  # three f16 products at 2.25 PFLOP/s are 0.75 of these
+    for b in bufs:
+        b.free()

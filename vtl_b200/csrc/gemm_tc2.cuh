@@ -725,10 +725,10 @@ int launch_pair(vtlb_ctx* ctx, const gemm::TmapSet& tm, const Epi& epi, int M, i
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN2 - 1) / BN2);
   int pairs = ctx->sm_count / 2;
   if (tiles < pairs) pairs = tiles;
-  // (a 3xTF32 launch behind a product on f16 planes is that product once more, if at all)
-  const bool timed = ctx->prof_on && ctx->prof_ev && ctx->prof_n < vtlb_ctx::kProfSlots &&
-                     !(KIND == gemm::KIND_TF32X3 && ho.unfit);
-  if (timed) cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n], ctx->stream);
+  // A product on f16 planes is two launches, of which one does the work: they are timed as one.
+  const bool timed = ctx->prof_on && ctx->prof_ev && ctx->prof_n < vtlb_ctx::kProfSlots;
+  const bool opens = KIND != gemm::KIND_TF32X3 || !ho.unfit, closes = KIND != gemm::KIND_F16X3;
+  if (timed && opens) cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n], ctx->stream);
   const int group_m = gemm::pick_group_m((M + 2 * BM - 1) / (2 * BM),
                                          (size_t)2 * BM * K * gemm::Traits<KIND>::ELEM * C::NOP);
   // When the final wave would fill at most half of the pairs, cut that many tiles into two half-K
@@ -750,7 +750,7 @@ int launch_pair(vtlb_ctx* ctx, const gemm::TmapSet& tm, const Epi& epi, int M, i
     kern<<<2 * pairs, NUM_THREADS, C::SMEM_TOTAL, ctx->stream>>>(tm, epi, M, N, K, group_m, a_chunk_k, split_tiles,
                                                                  (uint32_t*)ctx->ksplit_buf, ctx->ksplit_epoch,
                                                                  ctx->d_status, ho);
-  if (timed) {
+  if (timed && closes) {
     cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n + 1], ctx->stream);
     ctx->prof_n++;
     ctx->prof_flops += 2.0 * M * N * K;
