@@ -205,3 +205,28 @@ def test_time_of_a_product_that_f16_planes_cannot_hold(dev):
     assert ops / (ms * 1e-3) < 1.0e15  # three f16 products at 2.25 PFLOP/s are 0.75 of these
     for b in bufs:
         b.free()
+
+
+def test_switch_that_keeps_products_on_single_ctas():
+    """VTLB_F32_PAIR=0: two split passes and one product; else the f16 planes' two more launches."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import numpy as np
+from vtl_b200.capi import Device
+dev = Device(0)
+bufs = [dev.zeros(s) for s in ((2048, 256), (2048, 256), (2048, 2048))]
+n = dev.launch_count()
+dev.gemm_f32(False, True, 2048, 2048, 256, *bufs)
+dev.sync()
+print(dev.launch_count() - n)
+"""
+    got = {}
+    for pair in ("0", "1"):
+        root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+        p = subprocess.run([sys.executable, "-c", code], cwd=root, env={**os.environ, "VTLB_F32_PAIR": pair},
+                           capture_output=True, text=True, timeout=300)
+        assert p.returncode == 0, p.stderr
+        got[pair] = int(p.stdout)
+    assert got == {"0": 3, "1": 5}

@@ -542,7 +542,7 @@ int gemm_f32_impl(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
     };
     small = !over(C) && !(pre && over(pre));
   }
-  if (!small && !planes_in_or_out && gemm2::pair_worthwhile(ctx, M, N)) {
+  if (!small && !planes_in_or_out && f32::pair_product(ctx, M, N)) {
     // Large products: f16 planes on CTA pairs, twice the tensor rate of TF32 planes and half their bytes.  Planes
     // that come in or go out are TF32 ones, so products with those keep the 3xTF32 kernel.
     const int blocks = (K + gemm::kHalfBlock - 1) / gemm::kHalfBlock;

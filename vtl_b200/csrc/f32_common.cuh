@@ -106,6 +106,18 @@ inline int alloc_half_planes(vtlb_ctx* ctx, int rows_a, int rows_b, int K, size_
   return VTLB_OK;
 }
 
+// Large products run on CTA pairs, 256 x 256 tiles, on f16 planes where none come in or go out (f32.cu);
+// VTLB_F32_PAIR=0 keeps them on single CTAs and TF32 planes.
+inline bool pair_product(vtlb_ctx* ctx, int M, int N) {
+  static int env = -2;
+  if (env == -2) {
+    const char* e = getenv("VTLB_F32_PAIR");
+    env = e ? atoi(e) : -1;
+  }
+  return env != 0 && gemm2::pair_worthwhile(ctx, M, N);
+}
+
+// VTLB_F32_BN: columns of a single CTA's tile (64 or 128) instead of the rule below; pairs have 256.
 inline int bn_override() {
   static int v = -1;
   if (v < 0) {
@@ -186,13 +198,7 @@ int launch_tf32x3(vtlb_ctx* ctx, const Planes& p, int M, int N, int K, Epi epi, 
     if (N <= 64) bn = 64;
   }
   const uint64_t stride = (uint64_t)p.ld * 4;
-  // large problems: CTA pairs, 256 x 256 tiles (VTLB_F32_PAIR=0 keeps them on single CTAs)
-  static int pair_env = -2;
-  if (pair_env == -2) {
-    const char* e = getenv("VTLB_F32_PAIR");
-    pair_env = e ? atoi(e) : -1;
-  }
-  if (splits == 1 && pair_env != 0 && gemm2::pair_worthwhile(ctx, M, N)) {
+  if (splits == 1 && pair_product(ctx, M, N)) {
     if ((rc = encode_tf32_pair(ctx, &tm, p, M, N, K))) return rc;
     return gemm2::launch_pair<gemm::KIND_TF32X3, Epi>(ctx, tm, epi, M, N, K);
   }
