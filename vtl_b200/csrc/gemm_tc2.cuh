@@ -35,9 +35,6 @@ constexpr int BN2 = 256;      // columns of D per pair tile
 #define VTLB_PAIR_STAGES 6  // shared-memory ring depth of the INT8 pair kernel (tuning knob)
 #endif
 
-#ifndef VTLB_F16_CHUNK
-#define VTLB_F16_CHUNK 2
-#endif
 template <int KIND>
 struct Cfg {
   static constexpr int NOP = gemm::Traits<KIND>::NOP;                 // operand planes per side
@@ -56,7 +53,7 @@ struct Cfg {
   // costs three truncations per K step instead of one, still two orders inside the error bound.
   // The f16 planes close it every 2 stages = 128 elements (a stage holds twice the K).  At 4 stages the sums of
   // 4096 uniform products were off by 1.58e-6 of 64-bit ones where 3xTF32 leaves 1.08e-6; at 2 by 6.8e-7 (normal ones: 4.9e-7 against 9.2e-7).
-  static constexpr int CHUNK_KB = KIND == gemm::KIND_I8 ? 0 : KIND == gemm::KIND_F16X3 ? VTLB_F16_CHUNK : 4;
+  static constexpr int CHUNK_KB = KIND == gemm::KIND_I8 ? 0 : KIND == gemm::KIND_F16X3 ? 2 : 4;
   static constexpr int SCALE_KB = gemm::kHalfBlock * 2 / (int)ROW_BYTES;  // stages that share a scale (f16 planes)
   static_assert(KIND != gemm::KIND_F16X3 || SCALE_KB % CHUNK_KB == 0, "an accumulator has one scale");
 };
