@@ -70,3 +70,19 @@ def test_small_products_on_cuda_cores(dev, B, C, H, W, O, k, pad, relu, bias):
 def test_many_channels_on_tiny_planes(dev, B, C, H, O, k, pad):
     """The weights of all the channels that a CTA's threads could hold are more than a stage of shared memory."""
     _check(dev, B, C, H, H, O, k, pad, 1)
+
+
+@pytest.mark.parametrize("layer,direct", [
+    ((256, 3, 32, 32, 32, 3, 1), True), ((50, 1, 28, 28, 20, 5, 0), True), ((2, 4, 6, 6, 13, 1, 0), True),
+    ((50, 104, 18, 18, 214, 1, 0), False), ((31, 107, 28, 28, 189, 1, 0), False), ((125, 31, 14, 14, 54, 1, 0), False),
+    ((256, 32, 32, 32, 64, 3, 1), False),
+])
+def test_which_kernel_runs_forward(dev, layer, direct):
+    """1 x 1 layers that took up to three times as long on CUDA cores; first layers that take half as long there."""
+    B, C, H, W, O, k, pad = layer
+    bufs = [dev.zeros(s) for s in ((B, C, H, W), (O, C, k, k), (B, O, H + 2 * pad - k + 1, W + 2 * pad - k + 1))]
+    n = dev.launch_count()
+    dev.conv2d_fwd_f32(bufs[0], bufs[1], None, bufs[2], B, C, H, W, O, k, k, pad, pad, 1, 1)
+    assert (dev.launch_count() - n == 1) == direct
+    for b in bufs:
+        b.free()

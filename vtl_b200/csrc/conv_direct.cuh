@@ -283,30 +283,82 @@ inline int tile_rows(int Hd, int Wd) {
 constexpr int kMaxW = 128;        // output columns: a row of pixel groups fits a CTA, and the stage shared memory
 constexpr int kMaxTerms = 1600;   // terms of a sum up to which its error stays below the tensor-core kernels'
 
-// Microseconds, fitted to 116 measured products (forward and input gradient, batches 16 to 256, 1 to 64 channels,
-// 10 to 32 pixels, 3 x 3 and 5 x 5; mean error 17 %): products padded to whole threads, and the chain of stages.
-inline double direct_us(int B, int Cs, int Cd, int Hd, int Wd, int k) {
-  const int th = tile_rows(Hd, Wd), ct = wide(Cd) ? 8 : 4;
-  const double pixels = (double)B * ((Hd + th - 1) / th) * th * ((Wd + PX - 1) / PX) * PX;
-  return 5.7 + 0.0356e-6 * 2.0 * pixels * ((Cd + ct - 1) / ct * ct) * Cs * k * k + 0.13 * Cs * k;
+// The launch of a product: fills in the tiling fields of `p`; returns the bytes of shared memory.
+struct Launch {
+  long long tiles;   // of rows
+  int groups, CT;    // channel groups of CT
+  size_t smem;
+};
+inline Launch plan(vtlb_ctx* ctx, Params& p, int K) {
+  const int CT = wide(p.Cd) ? 8 : 4;
+  Launch l = {0, (p.Cd + CT - 1) / CT, CT, 0};
+  p.W4 = (p.Wd + PX - 1) / PX;
+  p.TH = tile_rows(p.Hd, p.Wd);
+  p.tiles_y = (p.Hd + p.TH - 1) / p.TH;
+  const int PG = p.TH * p.W4;
+  l.tiles = (long long)p.B * p.tiles_y;
+  p.CG = kThreads / PG < l.groups ? kThreads / PG : l.groups;
+  while (p.CG > 1 && l.tiles * ((l.groups + p.CG - 1) / p.CG) < 2 * ctx->sm_count) p.CG = (p.CG + 1) / 2;
+  p.pitch = (p.W4 * PX + K - 1 + 3) / 4 * 4;
+  // One source channel has to fit the stage.  On a tiny plane a CTA could hold the weights of hundreds of channels
+  // (256 groups of 8 on one pixel group); a single group takes 4 KB at most.
+  auto channel_bytes = [&] { return ((p.TH + K - 1) * p.pitch + K * K * p.CG * CT) * 4; };
+  while (p.CG > 1 && channel_bytes() > kStageBytes) p.CG = (p.CG + 1) / 2;
+  const int per_channel = channel_bytes();
+  p.Z = kThreads / (PG * p.CG);
+  if (p.Z > p.Cs) p.Z = p.Cs;
+  if (p.Z > 8) p.Z = 8;
+  p.CS = kStageBytes / per_channel;
+  if (p.CS > p.Cs) p.CS = p.Cs;
+  if (p.CS > p.Z) p.CS = p.CS / p.Z * p.Z;
+  l.smem = (size_t)p.CS * per_channel;
+  const size_t park = (size_t)(p.Z - 1) * PG * p.CG * CT * PX * 4;
+  if (park > l.smem) l.smem = park;
+  return l;
 }
-// The tensor-core kernels' (7 % mean error): waves of tiles of 128 pixels x 64 channels, each walking its K blocks of
-// 32; the gathered kernel stores planes of a size that is no multiple of 32 pixels value by value.
+
+// Microseconds.  3 x 3 and 5 x 5: fitted to 116 measured products (forward and input gradient, batches 16 to 256, 1 to 64
+// channels, 10 to 32 pixels; mean error 17 %): products padded to whole threads, and the chain of stages.  Of 234 more
+// (1 to 1024 images, 1 to 255 channels, 1 to 128 pixels) the rule below sent 2 to the slower kernel, by 16 and 30 %.
+// 1 x 1: fitted to 436 products over the wide range (16 %).  A window of one does so little with what it stages that
+// staging binds it: products of the threads that are there, the chain of source channels, what a CTA stages in each wave
+// of three per SM, and CTAs started.
+inline double direct_us(vtlb_ctx* ctx, int B, int Cs, int Cd, int Hd, int Wd, int k) {
+  if (k != 1) {
+    const int th = tile_rows(Hd, Wd), ct = wide(Cd) ? 8 : 4;
+    const double pixels = (double)B * ((Hd + th - 1) / th) * th * ((Wd + PX - 1) / PX) * PX;
+    return 5.7 + 0.0356e-6 * 2.0 * pixels * ((Cd + ct - 1) / ct * ct) * Cs * k * k + 0.13 * Cs * k;
+  }
+  Params p = {};
+  p.B = B, p.Cs = Cs, p.Cd = Cd, p.Hd = Hd, p.Wd = Wd;
+  const Launch l = plan(ctx, p, 1);
+  const double ctas = (double)l.tiles * ((l.groups + p.CG - 1) / p.CG);
+  const double products = ctas * p.TH * p.W4 * PX * p.CG * l.CT * Cs, staged = (double)Cs * (p.TH * p.pitch + p.CG * l.CT);
+  return 5.27 + 0.0954e-6 * products + 0.0371 * Cs + 0.767e-3 * ceil(ctas / (3 * ctx->sm_count)) * staged +
+         0.451 * ctas / ctx->sm_count;
+}
+// The tensor-core kernels' (7 % mean error, 1 x 1 11 %): waves of tiles of 128 pixels x 64 channels, each walking its K
+// blocks of 32; the gathered kernel stores planes of a size that is no multiple of 32 pixels value by value.
 inline double tensor_us(vtlb_ctx* ctx, const igemm::Geometry& g, const cslab::Tiling* slab, int Cd) {
   const double blocks_k = (g.K + 31) / 32, cols = (Cd + 63) / 64;
   const double tiles = cols * (slab ? (double)g.B * slab->tiles_per_img
                                     : (double)(((long long)g.B * g.Ho * g.Wo + 127) / 128));
-  const double waves = ceil(tiles / ctx->sm_count);
+  const double waves = ceil(tiles / ctx->sm_count), ragged = g.Ho * g.Wo % 32 ? Cd * tiles / ctx->sm_count : 0.0;
   if (slab) return 8.6 + waves * (2.8 + 0.273 * blocks_k);
-  return 9.8 + waves * (1.94 + 0.763 * blocks_k) + (g.Ho * g.Wo % 32 ? 0.126 * Cd * tiles / ctx->sm_count : 0.0);
+  if (g.kh == 1) return 6.9 + waves * (3.57 + 0.922 * blocks_k) + 0.0272 * ragged;
+  return 9.8 + waves * (1.94 + 0.763 * blocks_k) + 0.126 * ragged;
 }
+// Of the 436 products with a 1 x 1 window 323 run here, 10 of them slower than on tensor cores, by 42 % at most; the sum of
+// all is 10.3 ms, 28.4 on tensor cores alone, 10.1 with the better kernel each time.  With the 3 x 3 estimates it was
+// 11.6: they sent 50 x 104 x 18 x 18 -> 214 here (137 us, 42 on tensor cores).
 // At 256 x 3 x 32 x 32, 32 channels, 3 x 3: forward 24 us (40 on tensor cores), input gradient 55 (103); with 32 -> 64
 // channels 342 and 327 (106 and 190), which stay where they are.
 inline bool worthwhile(vtlb_ctx* ctx, const igemm::Geometry& g, const cslab::Tiling* slab, int Cd) {
   if (!mode() || !window_ok(g.kh, g.kw) || g.sy != 1 || g.sx != 1 || g.Wo > kMaxW || g.K > kMaxTerms ||
       (Cd + 3) / 4 > 65535)
     return false;
-  return mode() == 2 || 1.1 * direct_us(g.B, g.Cs, Cd, g.Ho, g.Wo, g.kh) < tensor_us(ctx, g, slab, Cd);
+  return mode() == 2 ||
+         (g.kh == 1 ? 1.2 : 1.1) * direct_us(ctx, g.B, g.Cs, Cd, g.Ho, g.Wo, g.kh) < tensor_us(ctx, g, slab, Cd);
 }
 // The weight gradient, likewise: rows of one image per SM on the tensor cores where that kernel applies
 // (cwgrad::usable), else the lowered product, bound by the patch matrix it writes.
@@ -322,42 +374,18 @@ inline bool wgrad_worthwhile(vtlb_ctx* ctx, int B, int C, int O, int Ho, int Wo,
   return mode() == 2 || 1.1 * direct < tensor;
 }
 
-template <int K, int CT>
-int launch_direct_t(vtlb_ctx* ctx, Params p) {
-  p.W4 = (p.Wd + PX - 1) / PX;
-  const int groups = (p.Cd + CT - 1) / CT;
-  p.TH = tile_rows(p.Hd, p.Wd);
-  p.tiles_y = (p.Hd + p.TH - 1) / p.TH;
-  const int PG = p.TH * p.W4;
-  const long long tiles = (long long)p.B * p.tiles_y;
-  p.CG = kThreads / PG < groups ? kThreads / PG : groups;
-  while (p.CG > 1 && tiles * ((groups + p.CG - 1) / p.CG) < 2 * ctx->sm_count) p.CG = (p.CG + 1) / 2;
-  p.pitch = (p.W4 * PX + K - 1 + 3) / 4 * 4;
-  // One source channel has to fit the stage.  On a tiny plane a CTA could hold the weights of hundreds of channels
-  // (256 groups of 8 on one pixel group); a single group takes 4 KB at most.
-  auto channel_bytes = [&] { return ((p.TH + K - 1) * p.pitch + K * K * p.CG * CT) * 4; };
-  while (p.CG > 1 && channel_bytes() > kStageBytes) p.CG = (p.CG + 1) / 2;
-  const int per_channel = channel_bytes();
-  p.Z = kThreads / (PG * p.CG);
-  if (p.Z > p.Cs) p.Z = p.Cs;
-  if (p.Z > 8) p.Z = 8;
-  p.CS = kStageBytes / per_channel;
-  if (p.CS > p.Cs) p.CS = p.Cs;
-  if (p.CS > p.Z) p.CS = p.CS / p.Z * p.Z;
-  size_t smem = (size_t)p.CS * per_channel;
-  const size_t park = (size_t)(p.Z - 1) * PG * p.CG * CT * PX * 4;
-  if (park > smem) smem = park;
+template <int K>
+int launch_direct_k(vtlb_ctx* ctx, Params p) {
+  const Launch l = plan(ctx, p, K);
   p.vec = p.Wd % 4 == 0 && vtlb_aligned16(p.dst) && (!p.pre || vtlb_aligned16(p.pre));
-  VTLB_CUDA(ctx, vtlb_launch_early(conv_direct_kernel<K, CT>, dim3((unsigned)tiles, (groups + p.CG - 1) / p.CG),
-                                   dim3(kThreads), smem, ctx->stream, p));
+  const dim3 grid((unsigned)l.tiles, (l.groups + p.CG - 1) / p.CG);
+  VTLB_CUDA(ctx, vtlb_launch_early(l.CT == 8 ? conv_direct_kernel<K, 8> : conv_direct_kernel<K, 4>, grid, dim3(kThreads),
+                                   l.smem, ctx->stream, p));
   VTLB_LAUNCHED(ctx);
   return VTLB_OK;
 }
-
 inline int launch_direct(vtlb_ctx* ctx, const Params& p, int K) {
-  if (K == 1) return wide(p.Cd) ? launch_direct_t<1, 8>(ctx, p) : launch_direct_t<1, 4>(ctx, p);
-  if (K == 3) return wide(p.Cd) ? launch_direct_t<3, 8>(ctx, p) : launch_direct_t<3, 4>(ctx, p);
-  return wide(p.Cd) ? launch_direct_t<5, 8>(ctx, p) : launch_direct_t<5, 4>(ctx, p);
+  return K == 1 ? launch_direct_k<1>(ctx, p) : K == 3 ? launch_direct_k<3>(ctx, p) : launch_direct_k<5>(ctx, p);
 }
 
 template <int K, int OT>
