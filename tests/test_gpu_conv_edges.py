@@ -86,3 +86,11 @@ def test_which_kernel_runs_forward(dev, layer, direct):
     assert (dev.launch_count() - n == 1) == direct
     for b in bufs:
         b.free()
+
+
+@pytest.mark.parametrize("B,C,H,W,O,k,pad", [
+    (2, 3, 11, 10, 4, 7, 3), (1, 2, 9, 8, 3, 7, 0), (2, 1, 7, 20, 5, 7, 6),   # 49 taps: more than the gathered kernel takes
+    (1, 2, 6, 7, 260, 3, 1), (2, 5, 5, 4, 90, 5, 2),                          # more (channel, tap) pairs than it takes
+])
+def test_unit_stride_on_the_lowered_route(dev, B, C, H, W, O, k, pad):
+    _check(dev, B, C, H, W, O, k, pad, 1)

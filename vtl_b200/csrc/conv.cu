@@ -210,11 +210,12 @@ __global__ void __launch_bounds__(256) grad_to_MO_split_kernel(const float* __re
 // kw = r, r + S, ..., at ow = j - (kw - r)/S, so no tap is tried in vain, nothing is divided per tap, and the
 // loads of a thread do not wait for one another.  One thread per column, trying every tap with a division each,
 // was bound by that arithmetic: 155 us for 32 x 64 x 56 x 56 at 3 x 3 / 2 (58 MB read, 26 MB written), 31 us so.
-// KT, ST: the square window and the stride at compile time; 0 = any (dilation too).
+// KT, ST: the square window and the stride at compile time; 0 = any (dilation too).  A unit stride with any window
+// (7 x 7, or more channels than the gathered kernel's table holds) needs no division either.
 template <int KT, int ST>
 __global__ void __launch_bounds__(256) col2im_gather_kernel(const float* __restrict__ dcolT, ConvDims d, int ldm,
                                                             float* __restrict__ dx) {
-  const int sw = ST ? ST : d.sw, khw = d.kh * d.kw;
+  const int sw = ST ? ST : d.sw, sh = ST ? ST : d.sh, khw = d.kh * d.kw;
   const int cells = (d.W + d.pw + sw - 1) / sw, n = d.H * cells;  // from q = 0: the cells left of pw hold nothing
   for (int plane = blockIdx.y; plane < d.B * d.C; plane += gridDim.y) {
     const int b = plane / d.C, ic = plane - b * d.C;
@@ -249,16 +250,16 @@ __global__ void __launch_bounds__(256) col2im_gather_kernel(const float* __restr
           if (iw >= 0 && iw < d.W) dst[(size_t)ih * d.W + iw] = s;
         }
       } else {
-        for (int r = 0; r < d.sw; ++r) {
-          const int iw = d.sw * j + r - d.pw;
+        for (int r = 0; r < sw; ++r) {
+          const int iw = sw * j + r - d.pw;
           if (iw < 0 || iw >= d.W) continue;
           float s = 0.0f;
           for (int kh = 0; kh < d.kh; ++kh) {
-            const int th = qh - kh * d.dh, oh = th / d.sh;
-            if (th < 0 || oh * d.sh != th || oh >= d.OH) continue;
+            const int th = qh - kh * d.dh, oh = th / sh;
+            if (th < 0 || oh * sh != th || oh >= d.OH) continue;
             for (int kw = 0; kw < d.kw; ++kw) {
-              const int tw = iw + d.pw - kw * d.dw, ow = tw / d.sw;
-              if (tw < 0 || ow * d.sw != tw || ow >= d.OW) continue;
+              const int tw = iw + d.pw - kw * d.dw, ow = tw / sw;
+              if (tw < 0 || ow * sw != tw || ow >= d.OW) continue;
               s = __fadd_rn(s, __ldg(src + (size_t)(kh * d.kw + kw) * ldm + oh * d.OW + ow));
             }
           }
@@ -662,7 +663,7 @@ int conv2d_bwd_impl(vtlb_ctx* ctx, const void* d_g, const void* d_x, const void*
     {
       const long long planes = (long long)B * C;
       const int n = H * ((W + pw + sw - 1) / sw);
-      auto kern = col2im_gather_kernel<0, 0>;
+      auto kern = sh == 1 && sw == 1 ? col2im_gather_kernel<0, 1> : col2im_gather_kernel<0, 0>;
       if (!dilated && sh == 2 && sw == 2 && kh == 3 && kw == 3) kern = col2im_gather_kernel<3, 2>;
       if (!dilated && sh == 2 && sw == 2 && kh == 5 && kw == 5) kern = col2im_gather_kernel<5, 2>;
       kern<<<dim3((n + 255) / 256 < 64 ? (n + 255) / 256 : 64, (unsigned)(planes < 32768 ? planes : 32768)), 256, 0,
