@@ -72,6 +72,45 @@ def test_many_channels_on_tiny_planes(dev, B, C, H, O, k, pad):
     _check(dev, B, C, H, H, O, k, pad, 1)
 
 
+# layer, and whether forward and input gradient may run on CUDA cores (a sum has at most 1600 terms there)
+FORCED = [
+    ((1, 1, 5, 5, 1, 5, 0), True, True), ((3, 3, 9, 7, 5, 3, 0), True, True), ((2, 2, 13, 11, 9, 5, 2), True, True),
+    ((2, 4, 6, 6, 13, 1, 0), True, True), ((2, 3, 8, 126, 12, 3, 2), True, True), ((1, 2, 3, 127, 6, 3, 2), False, True),
+    ((2, 3, 6, 5, 4, 1, 2), True, True), ((2, 1, 4, 4, 3, 5, 6), True, True), ((2, 64, 5, 5, 2, 5, 0), True, True),
+    ((2, 65, 5, 5, 2, 5, 0), False, True), ((16, 64, 14, 14, 80, 3, 1), True, True), ((40, 96, 28, 28, 70, 1, 0), True, True),
+]
+
+
+def forced(dev):
+    """Every layer of FORCED on the CUDA-core kernels (VTLB_CONV_DIRECT=2), which are one launch forward, one for the
+    input gradient; the tensor-core kernels have one more, which regroups the weights."""
+    for (B, C, H, W, O, k, pad), fwd, dx in FORCED:
+        _check(dev, B, C, H, W, O, k, pad, 1)
+        OH, OW = H + 2 * pad - k + 1, W + 2 * pad - k + 1
+        bufs = [dev.zeros(s) for s in ((B, C, H, W), (O, C, k, k), (B, O, OH, OW))]
+        dims = (B, C, H, W, O, k, k, pad, pad, 1, 1)
+        n = dev.launch_count()
+        dev.conv2d_fwd_f32(bufs[0], bufs[1], None, bufs[2], *dims)
+        assert (dev.launch_count() - n == 1) == fwd, (B, C, H, W, O, k, pad)
+        n = dev.launch_count()
+        dev.conv2d_bwd_f32(bufs[2], bufs[0], bufs[1], bufs[0], None, None, *dims)
+        assert (dev.launch_count() - n == 1) == dx, (B, C, H, W, O, k, pad)
+        for b in bufs:
+            b.free()
+
+
+def test_every_window_on_cuda_cores():
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = ("import sys; sys.path.insert(0, 'tests'); import test_gpu_conv_edges as t; from vtl_b200.capi import Device; "
+            "d = Device(0); t.forced(d); d.close()")
+    p = subprocess.run([sys.executable, "-c", code], cwd=root, env={**os.environ, "VTLB_CONV_DIRECT": "2"},
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
+
+
 @pytest.mark.parametrize("layer,direct", [
     ((256, 3, 32, 32, 32, 3, 1), True), ((50, 1, 28, 28, 20, 5, 0), True), ((2, 4, 6, 6, 13, 1, 0), True),
     ((50, 104, 18, 18, 214, 1, 0), False), ((31, 107, 28, 28, 189, 1, 0), False), ((125, 31, 14, 14, 54, 1, 0), False),
