@@ -84,7 +84,7 @@ int vtlb_profile_gemm_read(vtlb_ctx* ctx, double* total_ms, uint64_t* launches, 
  * collectives on the communication stream had finished: the exposed, not-overlapped part. */
 enum {
   VTLB_PHASE_GEMM = 0,       /* tensor-core GEMM / convolution launches */
-  VTLB_PHASE_SPLIT = 1,      /* f32 -> TF32 hi/lo operand planes */
+  VTLB_PHASE_SPLIT = 1,      /* f32 -> hi/lo operand planes (f16 or TF32) */
   VTLB_PHASE_OPTIMIZER = 2,  /* Adam / AdamW / SGD / RMSProp step */
   VTLB_PHASE_COMM_WAIT = 3,  /* compute stream waiting for collectives */
   VTLB_PHASE_ELEMENTWISE = 4,/* ReLU backward, bias-gradient column sums, loss kernels */
@@ -119,8 +119,14 @@ int vtlb_reserve_scratch(vtlb_ctx* ctx, size_t bytes);
 /* ---- f32 GEMM -------------------------------------------------------------
  * C[M,N] = op(A).op(B) (+ bias[N]) (ReLU).  op(A) is [M,K]: A is [M,K] row-major
  * when transA == 0, [K,M] when transA != 0; likewise B is [K,N] or, with transB,
- * [N,K].  Computed on tcgen05 tensor cores as a 3-pass TF32 split (hi.hi +
- * hi.lo + lo.hi) with f32 accumulation in tensor memory.
+ * [N,K].  Computed on tcgen05 tensor cores from hi/lo planes of the operands (hi.hi +
+ * hi.lo + lo.hi, f32 accumulation in tensor memory): TF32 planes, or, for products large enough for
+ * 256 x 256 tiles on pairs of SMs, f16 planes of block-scaled values, which hand the few elements they
+ * do not hold on to the epilogue and give the product back to TF32 planes where there are many.  Small
+ * products run on CUDA cores (below).  On every route, with n = K / 128 rounded up,
+ *     |C - A.B| <= (2^-21 + 48 * 2^-23 + n * 2^-24) * |A|.|B|   element by element
+ * before the bias (22 bits of every operand element, at most 48 truncations in an accumulator,
+ * n sums rounded to nearest), as long as no product or factor leaves the normal f32 range.
  * Replaces: la.matmul[f32] (la/la.v:38-55), gate_matmul
  * (autograd/gates_blas.v:6-23), compute.gemm_cuda as called from
  * autograd_cuda/device_session_d_cuda.v:43 and tensor_cuda_d_cuda.v:169, and
@@ -132,7 +138,8 @@ int vtlb_gemm_f32(vtlb_ctx* ctx, int transA, int transB, int M, int N, int K, co
  * from the caller's operands instead of the tensor-core path: at the size of a 784->256->10
  * MLP on a batch of 64 the call is bound by launch latency, not arithmetic.  Default 1.4e8, and
  * up to a few times that where K is long; a limit that is set is taken as it is;
- * 0 sends every product to the tensor cores.  Both paths meet the same error bound. */
+ * 0 sends every product to the tensor cores.  Above the limit C may lie over A or B (the operands are
+ * copied before C is written); up to the limit it may not. */
 int vtlb_set_small_gemm_limit(vtlb_ctx* ctx, double max_flops);
 
 /* ---- Linear layer ---------------------------------------------------------
@@ -155,9 +162,9 @@ int vtlb_linear_bwd_f32(vtlb_ctx* ctx, const void* d_G, const void* d_X, const v
                         int K);
 
 /* ---- the same two calls, with the operand planes handed from producer to consumer -----
- * The f32 products run as three TF32 MMAs on hi/lo planes of their operands (x = hi + lo).
- * vtlb_linear_fwd_f32 / _bwd_f32 write those planes in a pass of their own before every
- * product; in a deep network the same activation and gradient matrices are split again and
+ * With these the f32 products run as three TF32 MMAs on hi/lo planes of their operands (x = hi + lo).
+ * vtlb_linear_fwd_f32 / _bwd_f32 write planes in a pass of their own before every product (f16 ones
+ * for large products, at twice the rate: there they are the faster calls); in a deep network the same activation and gradient matrices are split again and
  * again (each is an operand of up to three products).  Here the GEMM that PRODUCES a matrix
  * also leaves its planes, from its epilogue, in the two layouts the consuming products read:
  *   "rows" planes of a matrix T[R,C]:  hi, lo as [R, vtlb_plane_ld(C)]   (T as the K-major operand)

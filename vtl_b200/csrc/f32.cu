@@ -3,12 +3,14 @@
 // nn/gates/layers/linear.v:69-79) on tcgen05 tensor cores.
 //
 // The reference multiplies in f64 and rounds once.  Here every f32 operand x is
-// split into two TF32 numbers, hi = tf32(x) and lo = tf32(x - hi), by a
-// memory-bound pass that also lays the operand out K-major (transposing when
-// the caller's layout is the other way round), and the GEMM issues three
-// kind::tf32 MMAs per K step (lo.hi + hi.lo + hi.hi).  The dropped lo.lo term
-// and the rounding of lo are ~2^-22 relative per product, well inside the
-// 1e-5*sqrt(K)*max|A|*max|B| bound.
+// split into hi and lo by a memory-bound pass that also lays the operand out
+// K-major (transposing when the caller's layout is the other way round), and the
+// GEMM issues three MMAs per K step (lo.hi + hi.lo + hi.hi).  hi and lo are TF32
+// numbers, or, where the product fills 256 x 256 tiles on CTA pairs, f16 numbers
+// of block-scaled values (struct HalfPlanes), at twice the tensor rate.  The
+// dropped lo.lo term and the rounding of lo are ~2^-22 relative per product, well
+// inside the 1e-5*sqrt(K)*max|A|*max|B| bound.  Small products run on CUDA cores
+// (small_product).
 #include "f32_common.cuh"
 
 namespace {

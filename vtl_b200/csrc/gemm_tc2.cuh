@@ -51,8 +51,9 @@ struct Cfg {
   // see gemm_tc.cuh).  With 256 columns per accumulator and two buffers there is no room in tensor
   // memory for a separate accumulator of the small cross terms: here they share the main one, which
   // costs three truncations per K step instead of one, still two orders inside the error bound.
-  // The f16 planes close it every 2 stages = 128 elements (a stage holds twice the K).  At 4 stages the sums of
-  // 4096 uniform products were off by 1.58e-6 of 64-bit ones where 3xTF32 leaves 1.08e-6; at 2 by 6.8e-7 (normal ones: 4.9e-7 against 9.2e-7).
+  // The f16 planes close it every 2 stages = 128 elements (a stage holds twice the K): sums of 4096 uniform products are
+  // off by 4.7e-7 of 64-bit ones, of normal ones by 2.3e-7, where 3xTF32 leaves 1.08e-6 and 9.2e-7.  (6.8e-7 and 4.9e-7
+  // with the cross terms among the hi.hi ones; so ordered, 4 stages left 1.58e-6 of uniform ones.)
   static constexpr int CHUNK_KB = KIND == gemm::KIND_I8 ? 0 : KIND == gemm::KIND_F16X3 ? 2 : 4;
   static constexpr int SCALE_KB = gemm::kHalfBlock * 2 / (int)ROW_BYTES;  // stages that share a scale (f16 planes)
   static_assert(KIND != gemm::KIND_F16X3 || SCALE_KB % CHUNK_KB == 0, "an accumulator has one scale");

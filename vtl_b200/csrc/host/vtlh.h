@@ -20,8 +20,9 @@ void* vtlh_session_ctx(vtlh_session* s); /* the vtlb_ctx* the session owns */
 int vtlh_session_comm_init(vtlh_session* s, int nranks, int rank, const void* id128);
 /* Seed of the layers' Kaiming-normal weight draws (restarts the per-layer counter). */
 int vtlh_session_set_seed(vtlh_session* s, unsigned long long seed);
-/* Whether large Linear layers hand TF32 operand planes from producer to consumer and fold the ReLU
- * backward into the gradient product (default on; off = every product splits its own operands). */
+/* Whether large Linear layers may hand TF32 operand planes from producer to consumer (by default none
+ * does, see the next call) and fold the ReLU backward into the gradient product (default on; off =
+ * every product splits its own operands and the ReLU backward is a pass of its own). */
 int vtlh_session_set_pass_planes(vtlh_session* s, int on);
 /* Smallest product (2*M*N*K flops) that hands its planes on; default infinity (see vtl_host.hpp). */
 int vtlh_session_set_plane_min_flops(vtlh_session* s, double flops);

@@ -121,7 +121,8 @@ class Session:
         _ck(self.lib.vtlh_session_set_seed(self.h, int(seed)))
 
     def set_pass_planes(self, on: bool):
-        """Producer-to-consumer hand-over of TF32 operand planes in large Linear layers (default on)."""
+        """Whether large Linear layers may hand TF32 operand planes on (see set_plane_min_flops: by default none does)
+        and fold the ReLU backward into the gradient product (default on)."""
         _ck(self.lib.vtlh_session_set_pass_planes(self.h, int(on)))
 
     def set_plane_min_flops(self, flops: float):
