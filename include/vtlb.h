@@ -123,7 +123,7 @@ int vtlb_reserve_scratch(vtlb_ctx* ctx, size_t bytes);
  * hi.lo + lo.hi, f32 accumulation in tensor memory): TF32 planes, or, for products large enough for
  * 256 x 256 tiles on pairs of SMs, f16 planes of block-scaled values, which hand the few elements they
  * do not hold on to the epilogue and give the product back to TF32 planes where there are many.  Small
- * products run on CUDA cores (below).  On every route, with n = K / 128 rounded up,
+ * products run on CUDA cores (below), in f32 throughout.  On the tensor cores, with n = K / 128 rounded up,
  *     |C - A.B| <= (2^-21 + 48 * 2^-23 + n * 2^-24) * |A|.|B|   element by element
  * before the bias (22 bits of every operand element, at most 48 truncations in an accumulator,
  * n sums rounded to nearest), as long as no product or factor leaves the normal f32 range.
